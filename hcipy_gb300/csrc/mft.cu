@@ -11,6 +11,7 @@
 #include "hx_common.cuh"
 #include "gemm_simt.cuh"
 #include "mft_tc.cuh"
+#include "plane_mft.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -28,6 +29,7 @@ struct hx_mft_plan {
     void* m2a = nullptr;  // nu x nx : exp(+i u x) wx[x]
     bool own_adjoint = false;
     hx::SplitMftPlan* split = nullptr;  // tensor-core operands (HX_PREC_SPLIT)
+    hx::PlaneMft* plane = nullptr;      // tensor-core operands of a plain plan (nullptr: CUDA cores alone)
     int schedule = HX_SCHEDULE_LATENCY;
 };
 
@@ -83,6 +85,7 @@ void free_plan(hx_mft_plan* p) {
         cudaFree(p->m2a);
     }
     hx::split_mft_destroy(p->split);
+    hx::plane_mft_destroy(p->plane);
     delete p;
 }
 
@@ -347,7 +350,7 @@ int run_small(int R, int K1, int K2, int C, typename hx::cplx<T>::type alpha, co
 
 template <typename T>
 int execute_t(const hx_mft_plan* p, int direction, int batch, const void* in_, void* out_, double are, double aim,
-              int epilogue, const void* mask, const void* src, void* ws_, cudaStream_t stream) {
+              int epilogue, const void* mask, const void* src, void* ws_, size_t ws_bytes, cudaStream_t stream) {
     using Cx = typename hx::cplx<T>::type;
     const Cx* in = (const Cx*)in_;
     Cx* out = (Cx*)out_;
@@ -360,10 +363,15 @@ int execute_t(const hx_mft_plan* p, int direction, int batch, const void* in_, v
     epi.kind = epilogue;
     epi.mask = (const Cx*)mask;
     epi.src = (const Cx*)src;
-    if (!tp) {
-        // small transforms: one launch (see mft_small_kernel)
-        const bool fwd = direction == HX_FORWARD;
-        const int R = fwd ? nv : ny, K1 = fwd ? ny : nv, K2 = fwd ? nx : nu, C = fwd ? nu : nx;
+    const size_t plane_bytes = hx::plane_mft_workspace_bytes(p->plane, direction, batch);
+    const bool plane = plane_bytes > 0 && ws_bytes >= plane_bytes;  // a caller with less scratch: the CUDA cores
+    const bool fwd = direction == HX_FORWARD;
+    const int R = fwd ? nv : ny, K1 = fwd ? ny : nv, K2 = fwd ? nx : nu, C = fwd ? nu : nx;
+    // Small transforms run in one launch (see mft_small_kernel).  complex128 products run on the float64 pipe there
+    // (two multiply-adds per clock and SM): 256^2 <- 128^2, 1.3e7 complex multiply-adds, takes 157 us of it against
+    // 40 us on the tensor cores; at 4e6 the one launch is the faster.
+    const double cmacs = (double)batch * ((double)K1 * K2 * C + (double)R * K1 * C);
+    if (!tp && !(plane && sizeof(T) == 8 && cmacs >= 8e6)) {
         if (small_form_ok<T>(R, K1, K2, C, batch, in, (long long)K1 * K2)) {
             const void* A = fwd ? p->m1f : direction == HX_BACKWARD ? p->m1b : p->m1a;
             const void* B = fwd ? p->m2f : direction == HX_BACKWARD ? p->m2b : p->m2a;
@@ -372,6 +380,9 @@ int execute_t(const hx_mft_plan* p, int direction, int batch, const void* in_, v
                                 stream);
         }
     }
+    if (plane)
+        return hx::plane_mft_execute(p->plane, direction, batch, in, out, are, aim, epilogue, mask, src, tp, ws_,
+                                     stream);
     if (direction == HX_FORWARD) {
         // T (batch*ny x nu) = in (batch*ny x nx) . M2f (nx x nu)
         HX_TRY(hx::cgemm_nn<T>(batch * ny, nu, nx, one, in, nx, 0, (const Cx*)p->m2f, nu, 0, T1, nu, 0, 1, stream, {},
@@ -391,7 +402,28 @@ int execute_t(const hx_mft_plan* p, int direction, int batch, const void* in_, v
     return hx::cgemm_nn<T>(batch * ny, nx, nu, alpha, T1, nu, 0, m2, nx, 0, out, nx, 0, 1, stream, epi, tp);
 }
 
+// Scratch of the Lyot chain with the transforms' scratch as `mft_bytes` counts it.
+size_t lyot_workspace_bytes(const hx_mft_plan* fpm, const hx_mft_plan* img, int batch,
+                            size_t (*mft_bytes)(const hx_mft_plan*, int, int)) {
+    if (!fpm || batch <= 0) return 0;
+    if (fpm->precision == HX_PREC_SPLIT)
+        return hx::split_lyot_workspace_bytes(fpm->split, img ? img->split : nullptr, batch);
+    const size_t es = fpm->esize;
+    size_t mft = std::max(mft_bytes(fpm, HX_FORWARD, batch), mft_bytes(fpm, HX_BACKWARD, batch));
+    if (img) mft = std::max(mft, mft_bytes(img, HX_FORWARD, batch));
+    const size_t focal = es * (size_t)batch * fpm->nu * fpm->nv;
+    const size_t pupil = es * (size_t)batch * fpm->nx * fpm->ny;
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    return up(focal) + up(pupil) + up(mft);
+}
+
 }  // namespace
+
+size_t hx::mft_least_workspace_bytes(const hx_mft_plan* p, int direction, int batch) {
+    if (!p || batch <= 0) return 0;
+    if (p->precision == HX_PREC_SPLIT) return hx::split_mft_workspace_bytes(p->split, direction, batch);
+    return p->esize * (size_t)batch * p->ny * p->nu;
+}
 
 extern "C" {
 
@@ -454,6 +486,9 @@ int hx_mft_plan_create(int nx, int ny, int nu, int nv, const double* x, const do
             if ((rc = gen_matrix(dtype, ny, nv, dy, dv, +1.0, dwy, nullptr, &p->m1a, stream))) break;
             if ((rc = gen_matrix(dtype, nu, nx, du, dx, +1.0, nullptr, dwx, &p->m2a, stream))) break;
         }
+        if (hx::plane_mft_fits(nx, ny, nu, nv, dtype) &&
+            hx::plane_mft_create(dtype, nx, ny, nu, nv, dx, dy, du, dv, dwx, dwy, dwu, dwv, stream, &p->plane) != HX_OK)
+            cudaGetLastError();  // no memory for the cut operands: the plan runs on the CUDA cores
     } while (false);
     cleanup();
     if (rc != HX_OK) {
@@ -465,10 +500,8 @@ int hx_mft_plan_create(int nx, int ny, int nu, int nv, const double* x, const do
 }
 
 size_t hx_mft_workspace_bytes(const hx_mft_plan* p, int direction, int batch) {
-    if (!p || batch <= 0) return 0;
-    size_t base = p->esize * (size_t)batch * p->ny * p->nu;
-    if (p->precision == HX_PREC_SPLIT) return hx::split_mft_workspace_bytes(p->split, direction, batch);
-    return base;
+    return std::max(hx::mft_least_workspace_bytes(p, direction, batch),
+                    p ? hx::plane_mft_workspace_bytes(p->plane, direction, batch) : (size_t)0);
 }
 
 int hx_mft_execute(const hx_mft_plan* p, int direction, int batch, const void* in, void* out, double are, double aim,
@@ -485,7 +518,7 @@ int hx_mft_execute_ex(const hx_mft_plan* p, int direction, int batch, const void
                  "hx_mft_execute: unknown direction %d", direction);
     HX_CHECK_ARG(batch >= 1, "hx_mft_execute: batch must be >= 1 (got %d)", batch);
     HX_CHECK_ARG(in != nullptr && out != nullptr, "hx_mft_execute: NULL field pointer");
-    const size_t need = hx_mft_workspace_bytes(p, direction, batch);
+    const size_t need = hx::mft_least_workspace_bytes(p, direction, batch);
     HX_CHECK_ARG(ws != nullptr && ws_bytes >= need, "hx_mft_execute: workspace of %zu bytes needed, %zu given", need,
                  ws_bytes);
     HX_CHECK_ARG(epilogue == HX_EPI_NONE || epilogue == HX_EPI_MUL || epilogue == HX_EPI_BABINET,
@@ -498,8 +531,8 @@ int hx_mft_execute_ex(const hx_mft_plan* p, int direction, int batch, const void
         return hx::split_mft_execute(p->split, direction, batch, in, HX_C64, out, HX_C64, are, aim, epilogue,
                                      (const float2*)mask, src, HX_C64, ws, ws_bytes, stream);
     if (p->dtype == HX_C64)
-        return execute_t<float>(p, direction, batch, in, out, are, aim, epilogue, mask, src, ws, stream);
-    return execute_t<double>(p, direction, batch, in, out, are, aim, epilogue, mask, src, ws, stream);
+        return execute_t<float>(p, direction, batch, in, out, are, aim, epilogue, mask, src, ws, ws_bytes, stream);
+    return execute_t<double>(p, direction, batch, in, out, are, aim, epilogue, mask, src, ws, ws_bytes, stream);
 }
 
 int hx_mft_execute_io(const hx_mft_plan* p, int direction, int batch, const void* in, int in_dtype, void* out,
@@ -540,16 +573,7 @@ int hx_mft_execute_phase(const hx_mft_plan* p, int batch, const void* in, const 
 }
 
 size_t hx_lyot_workspace_bytes(const hx_mft_plan* fpm, const hx_mft_plan* img, int batch) {
-    if (!fpm || batch <= 0) return 0;
-    if (fpm->precision == HX_PREC_SPLIT)
-        return hx::split_lyot_workspace_bytes(fpm->split, img ? img->split : nullptr, batch);
-    const size_t es = fpm->esize;
-    size_t mft = std::max(hx_mft_workspace_bytes(fpm, HX_FORWARD, batch), hx_mft_workspace_bytes(fpm, HX_BACKWARD, batch));
-    if (img) mft = std::max(mft, hx_mft_workspace_bytes(img, HX_FORWARD, batch));
-    const size_t focal = es * (size_t)batch * fpm->nu * fpm->nv;
-    const size_t pupil = es * (size_t)batch * fpm->nx * fpm->ny;
-    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    return up(focal) + up(pupil) + up(mft);
+    return lyot_workspace_bytes(fpm, img, batch, hx_mft_workspace_bytes);
 }
 
 int hx_lyot_execute(const hx_mft_plan* fpm, const hx_mft_plan* img, int batch, const void* e, int e_dtype,
@@ -563,7 +587,7 @@ int hx_lyot_execute(const hx_mft_plan* fpm, const hx_mft_plan* img, int batch, c
     HX_CHECK_ARG(!img || (img->nx == fpm->nx && img->ny == fpm->ny && img->precision == fpm->precision),
                  "hx_lyot_execute: the image plan must share the pupil grid and the precision of the mask plan");
     HX_CHECK_ARG(!img || image_out != nullptr, "hx_lyot_execute: image plan given without an image output");
-    const size_t need = hx_lyot_workspace_bytes(fpm, img, batch);
+    const size_t need = lyot_workspace_bytes(fpm, img, batch, hx::mft_least_workspace_bytes);
     HX_CHECK_ARG(ws != nullptr && ws_bytes >= need, "hx_lyot_execute: workspace of %zu bytes needed", need);
     if (hx::fault_injected("launch")) return HX_ERR_INJECTED;
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -595,7 +619,7 @@ int hx_lyot_execute(const hx_mft_plan* fpm, const hx_mft_plan* img, int batch, c
 
 int hx_mft_plan_status(const hx_mft_plan* p, int reset) {
     HX_CHECK_ARG(p != nullptr, "hx_mft_plan_status: plan is NULL");
-    if (p->precision != HX_PREC_SPLIT) return HX_OK;
+    if (p->precision != HX_PREC_SPLIT) return hx::plane_mft_status(p->plane, reset);
     return hx::split_mft_status(p->split, reset);
 }
 

@@ -28,6 +28,7 @@
 // start at zero.  Two calls whose kernels overlap on the GPU (different
 // streams, or different host threads without ordering) race on the array.
 #include "hx_common.cuh"
+#include "plane_mft.cuh"
 
 #include <cuda.h>
 
@@ -97,7 +98,7 @@ int hx_mft_execute_noalloc(const hx_mft_plan* plan, int direction, int batch, co
                            double alpha_re, double alpha_im, void* stream) {
     HX_CHECK_ARG(plan != nullptr, "hx_mft_execute_noalloc: plan is NULL");
     HX_CHECK_ARG(batch >= 1, "hx_mft_execute_noalloc: batch must be >= 1 (got %d)", batch);
-    const size_t need = hx_mft_workspace_bytes(plan, direction, batch);
+    const size_t need = hx::mft_least_workspace_bytes(plan, direction, batch);
     HX_CHECK_ARG(need <= (size_t)HX_MFT_NOALLOC_SCRATCH_BYTES,
                  "hx_mft_execute_noalloc: this transform needs %zu bytes of scratch for batch %d, more than the "
                  "%d-byte static scratch; use hx_mft_execute with a workspace, or a smaller batch",
