@@ -24,12 +24,13 @@
 // (below 2^-56 of the two scales), both under the rounding of a float64 product.
 //
 // Pipeline.  One CTA per 128 rows x BN real columns (BN = 128 for complex64, 64 for complex128, whose seven levels
-// take 448 of the 512 TMEM columns): warp 0 issues TMA boxes of all planes of a K step, warp 1 the MMAs, warps 2-9
+// take 448 of the 512 TMEM columns): warp 0 issues TMA boxes of all planes of a K step, warp 1 the MMAs, the others
 // drain.  Each accumulator has its own pair of barriers, so level l of the next partial sum starts as soon as level
 // l of this one is drained: complex64 alternates two sets of accumulators, complex128 drains its levels in the order
 // in which the next step's MMAs reach them.
-// With few tiles the CTAs of a thread-block cluster split K and add their partial sums, in rank order, through
-// distributed shared memory, each CTA finishing a slice of the columns.
+// With few tiles the CTAs of a thread-block cluster split K and add their partial sums in rank order, each CTA
+// finishing a slice of the columns.  The sums travel through L2 under the cluster's barrier: through distributed shared
+// memory they moved at 7 to 13 bytes per clock and SM.
 // All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word.
 #pragma once
 
@@ -42,21 +43,20 @@ namespace hx {
 namespace pg {
 
 constexpr int BM = 128;            // rows of A per tile (TMEM lanes)
-constexpr int NUM_THREADS = 320;   // TMA warp, MMA warp, 8 epilogue warps
-constexpr int EPI_THREADS = 256;
 constexpr uint64_t WAIT_LIMIT = 2000000000ull;
 constexpr int NAN_EXP = -(1 << 28);  // row exponent of a row that holds an infinity or a NaN (complex128)
 
 // Planes (NP), accumulators (LV), real columns per tile (BN), K' per stage (BK), accumulator sets (SETS), stages per
-// partial sum (CT) and partial sums per stage (PPS), pipeline stages (ST).
+// partial sum (CT) and partial sums per stage (PPS), pipeline stages (ST), epilogue threads (EPI: complex64 drains often
+// and little, complex128 seldom and much, and its conversions want warps).
 template <typename T> struct Shape;
 template <> struct Shape<float> {
-    static constexpr int NP = 2, LV = 1, BN = 128, BK = 64, SETS = 4, CT = 1, PPS = 2, ST = 3;
+    static constexpr int NP = 2, LV = 1, BN = 128, BK = 64, SETS = 4, CT = 1, PPS = 2, ST = 3, EPI = 256;
     using Acc = float;
     using Scale = float;
 };
 template <> struct Shape<double> {
-    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, SETS = 1, CT = 4, PPS = 1, ST = 2;
+    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, SETS = 1, CT = 4, PPS = 1, ST = 2, EPI = 512;
     struct __align__(16) Acc {
         long long hi, lo;  // value = hi 2^-38 + lo 2^-62 (times the scales)
     };
@@ -72,6 +72,9 @@ template <typename T> struct Layout {
     static constexpr int PIPE = S::ST * STAGE;
     static constexpr int SMEM = PIPE + 1024 + 1024;  // alignment slack; barriers, flags, column scales
     static constexpr int TN = S::BN / 2;            // complex columns per tile
+    static constexpr int THREADS = S::EPI + 64;     // TMA warp, MMA warp, epilogue warps
+    static constexpr int COLS = S::BN / (S::EPI / BM);  // real columns per epilogue thread
+    static constexpr int LD = COLS < 32 ? COLS : 32;    // columns per TMEM load
     static constexpr int NACC = S::SETS * S::LV;
     static constexpr int TMEM_COLS = 512;
     static_assert(NACC * S::BN <= TMEM_COLS, "the accumulators must fit TMEM");
@@ -94,9 +97,11 @@ struct PlaneArgs {
     long long ldo, out_z;   // element (m, n): out[field * out_z + n * ldo + row of the field]
     Cx* out;
     Cx alpha;
+    int alpha_kind;         // 0: 1, 1: real, 2: imaginary, 3: complex (told apart on the host, not on the float64 pipe)
     int epi;                // HX_EPI_*
     const Cx* mask;         // one field, indexed n * ldo + row
     const Cx* src;          // indexed like out
+    typename Shape<T>::Acc* parts;  // scratch of a K split: one tile's sums per CTA
     int* status;
 };
 
@@ -109,7 +114,9 @@ template <int ROW_BYTES> constexpr uint32_t desc_hi() {
     return ((8 * ROW_BYTES) >> 4) | (1u << 14) | ((ROW_BYTES == 128 ? 2u : 4u) << 29);
 }
 
-__device__ __forceinline__ void tmem_ld_32(uint32_t taddr, float* v) {
+template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v);
+template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, float* v) { ptx::tmem_ld_16(taddr, v); }
+template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float* v) {
     uint32_t r[32];
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
@@ -128,43 +135,43 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// (hi 2^24 + lo) 2^e rounded to float64 with integer operations (the float64 pipe issues two operations per clock
-// and SM): normalise to 64 bits, round to 53, place the exponent.
-__device__ __forceinline__ double fixed_to_double(long long hi, long long lo, int e) {
-    long long h = hi + (lo >> 24);
-    unsigned int l = (unsigned int)lo & 0xffffffu;
-    const bool neg = h < 0;
-    if (neg) {
-        h = l ? ~h : -h;
-        l = (0x1000000u - l) & 0xffffffu;
-    }
-    unsigned long long x = (unsigned long long)h;
-    int sh;
-    if (x == 0) {
-        if (l == 0) return 0.0;
-        sh = __clz((int)l) + 32;
-        x = (unsigned long long)l << sh;
-    } else {
-        const int lz = __clzll((long long)x);  // h is below 2^54
-        x = (x << lz) | (lz >= 24 ? (unsigned long long)l << (lz - 24) : (unsigned long long)(l >> (24 - lz)));
-        sh = lz - 24;
-    }
-    // the value is x 2^(e - sh) with the leading one of x at bit 63
-    const int be = e - sh + 63 + 1023;
-    const unsigned long long mant = (x >> 11) + ((x >> 10) & 1);  // 2^52 .. 2^53
-    if (be <= 0 || be >= 2046) {
-        // subnormal results and overflow: scale in two exact or correctly flushed steps
-        const double v = scalbn((double)mant, e - sh + 11);
-        return neg ? -v : v;
-    }
-    const unsigned long long bits = ((unsigned long long)(be - 1) << 52) + mant;  // a carry moves the exponent
-    return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0)));
+
+// (hi 2^24 + lo) 2^e rounded to float64 (|hi| < 2^53, |lo| < 2^48), with integer operations (the float64 pipe issues
+// about 1.6 operations per clock and SM) and without branches, so that the conversions of several columns overlap:
+// the sum's magnitude is normalised to a leading one at bit 63, rounded to 53 bits and given its exponent.  An exponent
+// out of float64's normal range sets `rare`; the caller then takes scaled_value.
+__device__ __forceinline__ double fixed_to_double(long long hi, long long lo, int e, bool& rare) {
+    const long long up = hi + (lo >> 24);            // units of 2^24, below 2^54
+    const unsigned int low = (unsigned int)lo << 8;  // the 24 bits below, left-aligned in 32
+    const unsigned int sign = (unsigned int)(up >> 63);
+    const unsigned long long mag = (unsigned long long)(up ^ (up >> 63)) + (low == 0 ? (sign & 1) : 0);
+    const unsigned int x2 = (unsigned int)(mag >> 32), x1 = (unsigned int)mag, x0 = low == 0 ? 0 : (low ^ sign) + (sign & 1);
+    // the leading non-zero word of x2 x1 x0 (x2 x1 in units of 2^24) and the two below it
+    const bool two = x2 != 0, one = x1 != 0;
+    const unsigned int y2 = two ? x2 : one ? x1 : x0, y1 = two ? x1 : one ? x0 : 0, y0 = two ? x0 : 0;
+    const int lz = __clz((int)y2);
+    const unsigned long long m =
+        ((unsigned long long)__funnelshift_l(y1, y2, lz) << 32 | __funnelshift_l(y0, y1, lz)) + 0x400;
+    // the exponent of the leading one, one more where the rounding carried out of the top
+    const int be = (two ? 63 : one ? 31 : -1) - lz + 24 + e + 1023 + (int)(m < 0x400);
+    rare |= y2 != 0 && (be < 1 || be > 2046);
+    const unsigned int fh = (unsigned int)(m >> 43) & 0xfffffu, fl = (unsigned int)(m >> 11);
+    const unsigned int top = fh | ((unsigned int)be << 20) | (sign & 0x80000000u);
+    return __hiloint2double(y2 == 0 ? 0 : (int)top, y2 == 0 ? 0 : (int)fl);
+}
+__device__ __noinline__ double scaled_value(long long hi, long long lo, int e) {
+    return scalbn(fma((double)hi, 0x1p24, (double)lo), e);
 }
 
-__device__ __forceinline__ float acc_value(const float& a, float rs, float cs) { return a * cs * rs; }
-__device__ __forceinline__ double acc_value(const Shape<double>::Acc& a, int re, int ce) {
+__device__ __forceinline__ float acc_value(const float& a, float rs, float cs, bool&) { return a * cs * rs; }
+__device__ __forceinline__ double acc_value(const Shape<double>::Acc& a, int re, int ce, bool& rare) {
+    rare |= re == NAN_EXP || ce == NAN_EXP;
+    return fixed_to_double(a.hi, a.lo, re + ce - 62, rare);
+}
+__device__ __forceinline__ float acc_rare(const float& a, float rs, float cs) { return a * cs * rs; }
+__device__ __forceinline__ double acc_rare(const Shape<double>::Acc& a, int re, int ce) {
     if (re == NAN_EXP || ce == NAN_EXP) return __longlong_as_double(0x7ff8000000000000ll);
-    return fixed_to_double(a.hi, a.lo, re + ce - 62);
+    return scaled_value(a.hi, a.lo, re + ce - 62);
 }
 
 __device__ __forceinline__ void acc_add(float& a, const float& b) { a += b; }
@@ -173,17 +180,21 @@ __device__ __forceinline__ void acc_add(Shape<double>::Acc& a, const Shape<doubl
     a.lo += b.lo;
 }
 
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+// Partial sums of the other CTAs of a K split travel through L2.
+__device__ __forceinline__ void put_part(float* p, float v) { __stcg(p, v); }
+__device__ __forceinline__ void put_part(Shape<double>::Acc* p, const Shape<double>::Acc& v) {
+    __stcg(reinterpret_cast<longlong2*>(p), make_longlong2(v.hi, v.lo));
 }
-__device__ __forceinline__ void st_cluster(uint32_t addr, const Shape<double>::Acc& v) {
-    asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(addr), "l"(v.hi), "l"(v.lo) : "memory");
+__device__ __forceinline__ float get_part(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ Shape<double>::Acc get_part(const Shape<double>::Acc* p) {
+    const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(p));
+    return {v.x, v.y};
 }
 
 // Running sums of one thread's columns.
 template <typename T> struct Sums;
 template <> struct Sums<float> {
-    static constexpr int COLS = Shape<float>::BN / 2;
+    static constexpr int COLS = Layout<float>::COLS;
     float tot[COLS], blk[COLS];
     int n = 0;
     __device__ __forceinline__ void clear() {
@@ -192,7 +203,7 @@ template <> struct Sums<float> {
     }
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) blk[j0 + j] += v[j];
+        for (int j = 0; j < Layout<float>::LD; ++j) blk[j0 + j] += v[j];
     }
     __device__ __forceinline__ void end_partial(bool last) {
         if ((++n & 15) != 0 && !last) return;
@@ -205,7 +216,7 @@ template <> struct Sums<float> {
     __device__ __forceinline__ float get(int j) const { return tot[j]; }
 };
 template <> struct Sums<double> {
-    static constexpr int COLS = Shape<double>::BN / 2;
+    static constexpr int COLS = Layout<double>::COLS;
     Shape<double>::Acc a[COLS];
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -215,7 +226,7 @@ template <> struct Sums<double> {
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
         constexpr int W = L < 4 ? 1 << (8 * (3 - L)) : 1 << (8 * (6 - L));
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < Layout<double>::LD; ++j) {
             const long long p = (long long)__float2int_rn(v[j]) * W;
             if (L < 4) a[j0 + j].hi += p;
             else a[j0 + j].lo += p;
@@ -225,8 +236,99 @@ template <> struct Sums<double> {
     __device__ __forceinline__ const Shape<double>::Acc& get(int j) const { return a[j]; }
 };
 
+// The finished columns of a tile: all of them, or with a K split over KS CTAs the ks-th of KS slices of its complex
+// columns, the CTA's own partial sums from shared memory and the others' from `others` (L2), added in rank order.
+// Lanes along the rows, so that the reads and the stores are contiguous; U columns at a time, their loads ahead of
+// their arithmetic.
+template <typename T, int KS>
+__device__ __forceinline__ void finish_columns(const PlaneArgs<T>& g, const typename Shape<T>::Acc* part_s,
+                                               const typename Shape<T>::Acc* others,
+                                               const typename Shape<T>::Scale* s_cs, typename Shape<T>::Scale rs,
+                                               int m0, int n_tile, int ks, int et) {
+    using Cx = typename cplx<T>::type;
+    using Acc = typename Shape<T>::Acc;
+    constexpr int TN = Layout<T>::TN, STEP = Shape<T>::EPI / BM, TNS = TN / KS;
+    constexpr int U = TNS / STEP < (sizeof(T) == 4 ? 4 : 2) ? TNS / STEP : (sizeof(T) == 4 ? 4 : 2);
+    static_assert(TNS % (STEP * U) == 0, "whole batches");
+    constexpr int PART = TN * 2 * BM;  // one CTA's partial sums
+    const int r = et & (BM - 1), m = m0 + r;
+    const bool mok = m < g.M;
+    const int z = mok ? m / g.rows_per_field : 0, y = mok ? m - z * g.rows_per_field : 0;
+    const Cx al = g.alpha;
+    const int kind = g.alpha_kind;
+    const Cx* mask = g.epi != HX_EPI_NONE ? g.mask : nullptr;
+#pragma unroll 1
+    for (int c = ks * TNS + et / BM; c < (ks + 1) * TNS; c += U * STEP) {
+        Acc re[U], im[U], xr[U][KS], xi[U][KS];
+        Cx e[U], mk[U], v[U];
+        bool rare = false;
+        long long o[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int at = (c + u * STEP) * 2 * BM + r;
+            if constexpr (KS > 1) {
+#pragma unroll
+                for (int sp = 0; sp < KS; ++sp) {
+                    if (sp == ks) continue;
+                    xr[u][sp] = get_part(others + sp * PART + at);
+                    xi[u][sp] = get_part(others + sp * PART + at + BM);
+                }
+            }
+            const int n = n_tile * TN + c + u * STEP;
+            const long long mo = (long long)n * g.ldo + y;
+            ok[u] = mok && n < g.N;
+            o[u] = (long long)z * g.out_z + mo;
+            if (ok[u] && g.epi == HX_EPI_BABINET) e[u] = g.src[o[u]];
+            if (ok[u] && mask) mk[u] = mask[mo];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int at = (c + u * STEP) * 2 * BM + r;
+            re[u] = part_s[at];
+            im[u] = part_s[at + BM];
+            if constexpr (KS > 1) {
+                const Acc own_r = re[u], own_i = im[u];
+#pragma unroll
+                for (int sp = 0; sp < KS; ++sp) {
+                    const Acc a = sp == ks ? own_r : xr[u][sp], b = sp == ks ? own_i : xi[u][sp];
+                    if (sp == 0) {
+                        re[u] = a;
+                        im[u] = b;
+                    } else {
+                        acc_add(re[u], a);
+                        acc_add(im[u], b);
+                    }
+                }
+            }
+            const auto cs = s_cs[c + u * STEP];
+            v[u] = make_c<T>(acc_value(re[u], rs, cs, rare), acc_value(im[u], rs, cs, rare));
+        }
+        if (rare) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const auto cs = s_cs[c + u * STEP];
+                v[u] = make_c<T>(acc_rare(re[u], rs, cs), acc_rare(im[u], rs, cs));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            Cx w = v[u];
+            if (kind == 1) w = make_c<T>(al.x * w.x, al.x * w.y);
+            else if (kind == 2) w = make_c<T>(-al.y * w.y, al.y * w.x);
+            else if (kind == 3) w = cmul(al, w);
+            if (g.epi == HX_EPI_BABINET) {
+                w.x = e[u].x - w.x;
+                w.y = e[u].y - w.y;
+            }
+            if (mask) w = cmul(w, mk[u]);
+            if (ok[u]) g.out[o[u]] = w;
+        }
+    }
+}
+
 template <typename T>
-__global__ void __launch_bounds__(NUM_THREADS, 1) plane_gemm_kernel(const __grid_constant__ PlaneArgs<T> g) {
+__global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const __grid_constant__ PlaneArgs<T> g) {
     using S = Shape<T>;
     using LY = Layout<T>;
     using Cx = typename cplx<T>::type;
@@ -265,7 +367,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) plane_gemm_kernel(const __grid
         }
         for (int a = 0; a < LY::NACC; ++a) {
             ptx::mbar_init(bar_ready(a), 1);
-            ptx::mbar_init(bar_drained(a), EPI_THREADS / 32);
+            ptx::mbar_init(bar_drained(a), S::EPI / 32);
         }
         ptx::mbar_init(bar_done, 1);
         *abort_flag = 0;
@@ -380,15 +482,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) plane_gemm_kernel(const __grid
         ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_done, 0, WAIT_LIMIT)) && ok;
         if (!ok && leader) give_up();
     }
-    // ---- warps 2..9: two per TMEM lane quarter, each one half of the columns ------------------------------------
+    // ---- warps 2 and up: two or four per TMEM lane quarter, each a slice of the columns ---------------------------------
     const bool epi = warp >= 2;
     const int et = threadIdx.x - 64;
     const int row = (warp & 3) * 32 + lane;
-    const int half = (warp - 2) >> 2;
+    const int slice = (warp - 2) >> 2;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    constexpr int COLS = S::BN / 2;
-    const int Sx = KS, TNS = LY::TN / Sx;
-    Acc* part_s = reinterpret_cast<Acc*>(smem);  // [split][complex column of the slice][re, im][row]
+    constexpr int COLS = LY::COLS;
+    Acc* part_s = reinterpret_cast<Acc*>(smem);  // [complex column][re, im][row]
+    // of a K split: the partial sums of the tile's CTAs, [CTA][complex column][re, im][row]
+    Acc* others = g.parts + ((long long)blockIdx.y * g.n_tiles + n_tile) * KS * (LY::TN * 2 * BM);
     if (epi) {
         Sums<T> sums;
         sums.clear();
@@ -406,9 +509,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) plane_gemm_kernel(const __grid
                 if (!live) return;
                 ptx::tc_fence_after();
 #pragma unroll
-                for (int j0 = 0; j0 < COLS; j0 += 32) {
-                    float v[32];
-                    tmem_ld_32(tmem + lane_base + a * S::BN + half * COLS + j0, v);
+                for (int j0 = 0; j0 < COLS; j0 += LY::LD) {
+                    float v[LY::LD];
+                    tmem_ld<LY::LD>(tmem + lane_base + a * S::BN + slice * COLS + j0, v);
                     sums.template add<l>(j0, v);
                 }
                 ptx::tc_fence_before();
@@ -427,65 +530,33 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) plane_gemm_kernel(const __grid
             if (!live) break;
             sums.end_partial(p == nparts - 1);
         }
-        if (Sx > 1) {
-            __syncwarp();
-            ptx::cluster_sync();  // every CTA's copies and MMAs are complete: the pipeline buffers are free
-        } else {
-            ptx::named_barrier(1, EPI_THREADS);
-        }
+        // every warp has seen the last accumulators, so this CTA's copies and MMAs are complete
+        ptx::named_barrier(1, S::EPI);
         if (live) {
+            constexpr int LOG_TN = LY::TN == 64 ? 6 : 5;
+            static_assert(1 << LOG_TN == LY::TN, "complex columns per tile");
+            Acc* mine = others + (long long)ks * LY::TN * 2 * BM;
 #pragma unroll
             for (int j = 0; j < COLS; ++j) {
-                const int c = half * COLS + j;                    // real column of the tile
-                const int cc = (c >> 4) * 8 + (c & 7), ri = (c >> 3) & 1;
-                const int owner = cc / TNS, ccl = cc - owner * TNS;
-                Acc* dst = part_s + ((ks * TNS + ccl) * 2 + ri) * BM + row;
-                if (owner == ks) *dst = sums.get(j);
-                else st_cluster(ptx::map_shared_rank(ptx::smem_addr(dst), (uint32_t)owner), sums.get(j));
+                const int c = slice * COLS + j;  // real column of the tile
+                const int cc = (c >> 4) * 8 + (c & 7);
+                const int at = (cc * 2 + ((c >> 3) & 1)) * BM + row;
+                if ((cc * KS) >> LOG_TN == ks) part_s[at] = sums.get(j);
+                else put_part(mine + at, sums.get(j));
             }
         }
-    } else if (Sx > 1) {
-        __syncwarp();
-        ptx::cluster_sync();
     }
-    if (Sx > 1) {
+    if (KS > 1) {
         __syncwarp();
-        ptx::cluster_sync();  // every partial sum is in place
+        ptx::cluster_sync();  // every CTA's partial sums are written (release and acquire cover L2 too)
     }
     if (epi) {
-        if (Sx == 1) ptx::named_barrier(1, EPI_THREADS);
-        const int r = et & (BM - 1), m = m0 + r;
-        if (m < g.M && *abort_flag == 0) {
-            const int z = m / g.rows_per_field, y = m - z * g.rows_per_field;
-            const int n0 = n_tile * LY::TN + ks * TNS;
-            const Cx al = g.alpha;
-            const bool imag_alpha = al.x == T(0), real_alpha = al.y == T(0);
-            const Cx* mask = g.epi != HX_EPI_NONE ? g.mask : nullptr;
-            const int step = EPI_THREADS / BM;
-#pragma unroll(sizeof(T) == 4 ? 8 : 4)
-            for (int cc = et / BM; cc < TNS; cc += step) {
-                const int n = n0 + cc;
-                if (n >= g.N) break;
-                const long long o = (long long)z * g.out_z + (long long)n * g.ldo + y;
-                const long long mo = (long long)n * g.ldo + y;
-                Acc re = part_s[(cc * 2) * BM + r], im = part_s[(cc * 2 + 1) * BM + r];
-                for (int sp = 1; sp < Sx; ++sp) {
-                    acc_add(re, part_s[((sp * TNS + cc) * 2) * BM + r]);
-                    acc_add(im, part_s[((sp * TNS + cc) * 2 + 1) * BM + r]);
-                }
-                const auto cs = s_cs[ks * TNS + cc];
-                Cx v = make_c<T>(acc_value(re, rs, cs), acc_value(im, rs, cs));
-                if (real_alpha) v = al.x == T(1) ? v : make_c<T>(al.x * v.x, al.x * v.y);
-                else if (imag_alpha) v = make_c<T>(-al.y * v.y, al.y * v.x);
-                else v = cmul(al, v);
-                if (g.epi == HX_EPI_BABINET) {
-                    const Cx e = g.src[o];
-                    v.x = e.x - v.x;
-                    v.y = e.y - v.y;
-                }
-                if (mask) v = cmul(v, mask[mo]);
-                g.out[o] = v;
-            }
+        if (KS == 1) ptx::named_barrier(1, S::EPI);
+        if (*abort_flag == 0) {
+            if (KS == 1) finish_columns<T, 1>(g, part_s, others, s_cs, rs, m0, n_tile, 0, et);
+            else if (KS == 2) finish_columns<T, 2>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+            else if (KS == 4) finish_columns<T, 4>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+            else finish_columns<T, 8>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
         }
     }
     ptx::tc_fence_before();

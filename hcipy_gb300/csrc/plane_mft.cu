@@ -340,7 +340,7 @@ template <typename T> bool cluster_ok(int ks) {
     if (!cache[dev][ks]) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ks);
-        cfg.blockDim = dim3(NUM_THREADS);
+        cfg.blockDim = dim3(Layout<T>::THREADS);
         cfg.dynamicSmemBytes = Layout<T>::SMEM;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -350,19 +350,21 @@ template <typename T> bool cluster_ok(int ks) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        const bool ok = cudaOccupancyMaxActiveClusters(&n, plane_gemm_kernel<T>, &cfg) == cudaSuccess && n > 0;
+        const bool ok = cudaFuncSetAttribute(plane_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             Layout<T>::SMEM) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, plane_gemm_kernel<T>, &cfg) == cudaSuccess && n > 0;
         cudaGetLastError();
         cache[dev][ks] = ok ? 1 : 2;
     }
     return cache[dev][ks] == 1;
 }
 
-// CTAs along K per tile: enough to occupy the SMs, each with at least two partial sums of complex128 (256 terms of
-// K') or eight of complex64 (512 terms), below which the exchange costs more than the shorter chain saves.
+// CTAs along K per tile: enough to occupy the SMs, each with at least one partial sum of complex128 (128 terms of K')
+// or four stages of complex64 (256 terms), below which the exchange costs more than the shorter chain saves.
 template <typename T> int k_split(long long tiles, int ktiles, bool throughput) {
     if (throughput) return 1;
     const int parts = (ktiles + Shape<T>::CT - 1) / Shape<T>::CT;
-    const int least = sizeof(T) == 4 ? 8 : 2;
+    const int least = sizeof(T) == 4 ? 4 : 1;
     for (int ks : {8, 4, 2})
         if (tiles * ks <= num_sms() && parts / ks >= least && cluster_ok<T>(ks)) return ks;
     return 1;
@@ -384,6 +386,7 @@ template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const 
     }
     g.M = (int)a.rows;
     g.N = b.n;
+    g.alpha_kind = g.alpha.y == 0 ? (g.alpha.x == 1 ? 0 : 1) : g.alpha.x == 0 ? 2 : 3;
     g.row_scale = (const typename Shape<T>::Scale*)a.scale;
     g.col_scale = (const typename Shape<T>::Scale*)b.scale;
     g.ktiles = a.kpitch / Shape<T>::BK;
@@ -393,7 +396,7 @@ template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const 
     TraceScope trace(HX_TRACE_SIMT_GEMM, cmacs, st);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(g.n_tiles * g.ksplit), m_tiles);
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(Layout<T>::THREADS);
     cfg.dynamicSmemBytes = LY::SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -431,6 +434,7 @@ Dims dims_of(const PlaneMft* p, int direction) {
 template <typename T> struct Pass {
     PlaneMat s1, s2;
     void* t = nullptr;
+    void* parts = nullptr;  // partial sums of a K split
     size_t bytes = 0;
     int fields = 1;
 };
@@ -442,6 +446,12 @@ template <typename T> size_t carve_pass(void* ws, const Dims& d, int fields, Pas
     carve_mat<T>(c, q.s1, r1, r1, d.K2);
     q.t = c.take(2 * sizeof(T) * (size_t)r2 * d.K1);
     carve_mat<T>(c, q.s2, r2, r2, d.K1);
+    auto part_bytes = [&](const PlaneMat& a, int N) {
+        const long long tiles = (long long)ceil_div(a.rows, BM) * ceil_div(N, Layout<T>::TN);
+        const int ks = k_split<T>(tiles, a.kpitch / Shape<T>::BK, false);
+        return ks > 1 ? (size_t)tiles * ks * Layout<T>::TN * 2 * BM * sizeof(typename Shape<T>::Acc) : (size_t)0;
+    };
+    q.parts = c.take(std::max(part_bytes(q.s1, d.C), part_bytes(q.s2, d.R)));
     q.bytes = c.off + 256;
     q.fields = fields;
     if (out) *out = q;
@@ -526,6 +536,7 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
         g1.out = (Cx*)q.t;
         g1.alpha = make_c<T>(T(1), T(0));
         g1.epi = HX_EPI_NONE;
+        g1.parts = (typename Shape<T>::Acc*)q.parts;
         g1.status = p->status;
         HX_TRY(launch_gemm<T>(g1, q.s1, p->rgt[direction], throughput, (double)nb * d.K1 * d.K2 * d.C, st));
         HX_TRY(launch_rows<T>(q.t, (long long)nb * d.C, d.K1, q.s2, st));
@@ -539,6 +550,7 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
         g2.epi = epilogue;
         g2.mask = (const Cx*)mask;
         g2.src = src ? (const Cx*)src + b0 * oplane : nullptr;
+        g2.parts = (typename Shape<T>::Acc*)q.parts;
         g2.status = p->status;
         HX_TRY(launch_gemm<T>(g2, q.s2, p->lft[direction], throughput, (double)nb * d.R * d.K1 * d.C, st));
     }
