@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
     long long* s_maskoff = reinterpret_cast<long long*>(extra + 2176);     // mask offset of the row
     unsigned int* s_rowmax = reinterpret_cast<unsigned int*>(extra + 3200);  // EMB: row maxima of the tile
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);  // warp-uniform
     const int lane = threadIdx.x & 31;
     // the K-splits of a tile are consecutive CTAs when they form a cluster, else n_tiles apart
     const int n_tile = g.cluster ? blockIdx.x / g.ksplit : blockIdx.x % g.n_tiles;
@@ -387,7 +387,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const uint32_t smem_base = ptx::smem_addr(smem);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -416,42 +417,45 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                     raise_status(g.status, abort_flag);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN);
-            // (A slice, B slice, level) of the kept products; the first product of a level starts it.
-            constexpr int NPROD = 8;
-            const int pa[NPROD] = {0, 0, 1, 0, 1, 2, 1, 2};
-            const int pb[NPROD] = {0, 1, 0, 2, 1, 0, 2, 1};
-            const int pl[NPROD] = {0, 1, 1, 2, 2, 2, 3, 3};
-            const int first[NPROD] = {1, 1, 0, 1, 0, 0, 1, 0};
-            for (int i = 0; i < nkt; ++i) {
-                if (*abort_flag) break;
-                const int s = i % STAGES;
-                const int u = i / STAGES;
-                if (!ptx::mbar_wait_bounded(bar_full(s), u & 1, WAIT_LIMIT)) {
-                    raise_status(g.status, abort_flag);
-                    break;
-                }
-                ptx::tc_fence_after();
-                const uint32_t a0 = ptx::smem_addr(smem + s * T::STAGE_BYTES);
-                const uint32_t b0 = a0 + A_STAGE_BYTES;
+        // The whole warp runs this branch with only the instructions themselves under the elected lane: issued from a
+        // one-lane branch, with 64-bit descriptors built for each, an MMA took 79 clocks of the issuing thread where
+        // the 128-column product itself takes 64.
+        constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN);
+        // descriptors of a K-major operand with 128-byte swizzle: 8-row groups 1024 B apart, version 1, swizzle mode 2
+        constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+        const bool leader = ptx::elect_one();
+        // (A slice, B slice, level) of the kept products; the first product of a level starts it.
+        constexpr int NPROD = 8;
+        const int pa[NPROD] = {0, 0, 1, 0, 1, 2, 1, 2};
+        const int pb[NPROD] = {0, 1, 0, 2, 1, 0, 2, 1};
+        const int pl[NPROD] = {0, 1, 1, 2, 2, 2, 3, 3};
+        const int first[NPROD] = {1, 1, 0, 1, 0, 0, 1, 0};
+        bool ok = true;
+        for (int i = 0; i < nkt; ++i) {
+            const int s = i % STAGES;
+            const int u = i / STAGES;
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, WAIT_LIMIT));
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint32_t a0 = (((smem_base + s * T::STAGE_BYTES) & 0x3FFFF) >> 4) | (1u << 16);
+            const uint32_t b0 = a0 + (A_STAGE_BYTES >> 4);
 #pragma unroll
-                for (int kk = 0; kk < BK / 16; ++kk) {
+            for (int kk = 0; kk < BK / 16; ++kk) {
 #pragma unroll
-                    for (int p = 0; p < NPROD; ++p) {
-                        const uint64_t ad = ptx::umma_desc_sw128(a0 + pa[p] * A_PLANE_BYTES + kk * 32);
-                        const uint64_t bd = ptx::umma_desc_sw128(b0 + pb[p] * T::B_PLANE_BYTES + kk * 32);
-                        const uint32_t acc = (i > 0 || kk > 0 || !first[p]) ? 1u : 0u;
-                        ptx::umma_f16(tmem + pl[p] * BN, ad, bd, idesc, acc);
-                    }
+                for (int p = 0; p < NPROD; ++p) {
+                    if (leader)
+                        ptx::umma_f16_lo(tmem + pl[p] * BN, a0 + ((pa[p] * A_PLANE_BYTES + kk * 32) >> 4),
+                                         b0 + ((pb[p] * T::B_PLANE_BYTES + kk * 32) >> 4), desc_hi, idesc,
+                                         i == 0 && kk == 0 && first[p]);
                 }
-                ptx::umma_commit(bar_empty(s));
             }
-            // Arrives once every MMA issued above has completed (at once if none was issued); TMEM is
-            // released only after that.
-            ptx::umma_commit(bar_accum);
-            if (!ptx::mbar_wait_bounded(bar_accum, 0, WAIT_LIMIT)) raise_status(g.status, abort_flag);
+            if (leader) ptx::umma_commit(bar_empty(s));
         }
+        // Arrives once every MMA issued above has completed (at once if none was issued); TMEM is
+        // released only after that.
+        if (leader) ptx::umma_commit(bar_accum);
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_accum, 0, WAIT_LIMIT)) && ok;
+        if (!ok && leader) raise_status(g.status, abort_flag);
     }
     // ---- epilogue: warps 2..9, two per TMEM lane quarter (each takes every other 16-column chunk) ----------
     constexpr int EPI = NUM_THREADS - 64;

@@ -82,30 +82,9 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);  // start address
-    d |= (uint64_t)(16 >> 4) << 16;           // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset: next 8-row group
-    d |= (uint64_t)1 << 46;                   // descriptor version
-    d |= (uint64_t)2 << 61;                   // 128-byte swizzle
-    return d;
-}
-
 // Instruction descriptor of kind::f16 with F16 A/B, F32 accumulator, both operands K-major.
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n) {
     return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 
 // True in one lane of a fully active warp.  Code that issues MMAs runs in the whole warp with only the instruction
@@ -121,8 +100,8 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
-// umma_f16 with the descriptors' low words (the start addresses, which alone change between MMAs) and their common
-// high word, accumulating unless `start`.
+// One kind::f16 MMA.  The operands' shared-memory descriptors come as their low words (start address in units of 16
+// bytes, which alone changes between MMAs) and a common high word; accumulates unless `start`.
 __device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc,
                                             bool start) {
     asm volatile(
