@@ -69,14 +69,18 @@ int launch_shape(int M, const std::vector<int>& radices, int nlines, int batch, 
         lpc = (int)std::max<long long>(std::min<long long>(lpc, std::max<long long>(lines_needed, min_lines)), 1);
     }
     lpc = std::min(lpc, nlines);
-    int thr = 32;
     const int ppt = mixed ? Ppt<T, true>::value : Ppt<T, false>::value;
-    for (int R : radices) {
-        const int bpt = std::max(1, ppt / R);
-        const int need = (lpc * (M / R) + bpt - 1) / bpt;
-        thr = std::max(thr, need);
-    }
-    thr = ((thr + 31) / 32) * 32;
+    auto threads_for = [&](int lines) {
+        int need = 32;
+        for (int R : radices) {
+            const int bpt = std::max(1, ppt / R);
+            need = std::max(need, (lines * (M / R) + bpt - 1) / bpt);
+        }
+        return (need + 31) / 32 * 32;
+    };
+    // a radix above the points a thread holds takes a thread per butterfly: fewer lines (300 = 4 5 5 3 in float64)
+    while (lpc > 1 && threads_for(lpc) > kFftThreads) --lpc;
+    const int thr = threads_for(lpc);
     if (thr > kFftThreads) {
         set_error("internal: FFT launch needs %d threads", thr);
         return HX_ERR_UNSUPPORTED;
@@ -123,28 +127,18 @@ int run_line_m(const LineArgs<T>& a, int threads, size_t smem, int sign, bool co
                     : launch_line<T, 1, false, MIXED>(a, threads, smem, batch, s);
 }
 
-// Threads per CTA of the register-resident power-of-two kernel: 512.  HX_FFT_P2_THREADS (256 or 512) and
-// HX_FFT_P2_THREADS_LF (256, 512 or 1024, strided lines) override it (tuning).
-int p2_threads(bool lf) {
-    static int v[2] = {0, 0};
-    if (!v[lf]) {
-        const char* e = getenv(lf ? "HX_FFT_P2_THREADS_LF" : "HX_FFT_P2_THREADS");
-        const int x = e ? atoi(e) : 0;
-        v[lf] = (x == 256 || x == 512 || (x == 1024 && lf)) ? x : 512;
-    }
-    return v[lf];
-}
-
-template <int N, int SIGN, bool LF>
+template <int N, int SIGN, bool LF, bool CONV>
 int launch_p2(const LineArgs<float>& a0, int batch, cudaStream_t stream) {
     using P = Pow2Shape<N>;
     LineArgs<float> a = a0;
-    const int lpc = std::max(1, std::min(p2_threads(LF) / P::T, a.nlines));
+    int lpc = P::template lines<LF>();
+    while (lpc > 1 && lpc / 2 >= a.nlines) lpc /= 2;  // a power of two: lines of a CTA are told apart by masks
     a.lines_per_cta = lpc;
-    const size_t smem = sizeof(float2) * (size_t)lpc * P::PITCH;
+    const size_t smem = sizeof(float2) * (size_t)lpc * P::template pitch<LF>();
     static bool configured = false;
     if (!configured) {
-        cudaFuncSetAttribute(fft_pow2_kernel<N, SIGN, LF>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(fft_pow2_kernel<N, SIGN, LF, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             227 * 1024);
         configured = true;
     }
     dim3 grid((a.nlines + lpc - 1) / lpc, batch);
@@ -153,28 +147,36 @@ int launch_p2(const LineArgs<float>& a0, int batch, cudaStream_t stream) {
         return HX_ERR_UNSUPPORTED;
     }
     TraceScope trace(HX_TRACE_FFT, (double)a.nlines * (a.in_count + a.out_count) * batch * sizeof(float2), stream);
-    fft_pow2_kernel<N, SIGN, LF><<<grid, lpc * P::T, smem, stream>>>(a);
+    fft_pow2_kernel<N, SIGN, LF, CONV><<<grid, lpc * P::T, smem, stream>>>(a);
     return launch_status("fft_pow2_kernel");
 }
 
 template <int N>
-int run_p2_n(const LineArgs<float>& a, int sign, int batch, cudaStream_t s) {
+int run_p2_n(const LineArgs<float>& a, int sign, bool conv, int batch, cudaStream_t s) {
     const bool lf = a.in_es != 1;
-    if (sign < 0) return lf ? launch_p2<N, -1, true>(a, batch, s) : launch_p2<N, -1, false>(a, batch, s);
-    return lf ? launch_p2<N, 1, true>(a, batch, s) : launch_p2<N, 1, false>(a, batch, s);
+    if (conv) {
+        if (sign > 0) return -1;  // a convolution runs forward first
+        return lf ? launch_p2<N, -1, true, true>(a, batch, s) : launch_p2<N, -1, false, true>(a, batch, s);
+    }
+    if (sign < 0)
+        return lf ? launch_p2<N, -1, true, false>(a, batch, s) : launch_p2<N, -1, false, false>(a, batch, s);
+    return lf ? launch_p2<N, 1, true, false>(a, batch, s) : launch_p2<N, 1, false, false>(a, batch, s);
 }
 
-// The register-resident kernel takes complex64 power-of-two lines of 256 to 4096 points without Bluestein chirps
-// or a spectrum multiply, whose input and output lines are both contiguous or both strided; -1 otherwise.
+// The register-resident kernel takes complex64 power-of-two lines of 256 to 4096 points without Bluestein chirps,
+// with or without a spectrum multiply, whose input and output lines are both contiguous or both strided (by less than
+// 2^31 elements); -1 otherwise.
 int run_p2(const LineArgs<float>& a, int sign, bool conv, int batch, cudaStream_t s) {
-    if (conv || !a.tws || a.chirp_in || a.chirp_out || a.n_log != a.M || (a.in_es != 1) != (a.out_es != 1))
+    if (!a.tws || a.chirp_in || a.chirp_out || a.n_log != a.M || a.out_mod != a.M ||
+        (a.in_es != 1) != (a.out_es != 1) ||
+        std::max(std::max(a.in_es, a.out_es), std::max(a.mid_es, a.post_es)) > 0x7fffffffll)
         return -1;
     switch (a.M) {
-        case 256: return run_p2_n<256>(a, sign, batch, s);
-        case 512: return run_p2_n<512>(a, sign, batch, s);
-        case 1024: return run_p2_n<1024>(a, sign, batch, s);
-        case 2048: return run_p2_n<2048>(a, sign, batch, s);
-        case 4096: return run_p2_n<4096>(a, sign, batch, s);
+        case 256: return run_p2_n<256>(a, sign, conv, batch, s);
+        case 512: return run_p2_n<512>(a, sign, conv, batch, s);
+        case 1024: return run_p2_n<1024>(a, sign, conv, batch, s);
+        case 2048: return run_p2_n<2048>(a, sign, conv, batch, s);
+        case 4096: return run_p2_n<4096>(a, sign, conv, batch, s);
         default: return -1;
     }
 }
@@ -490,6 +492,19 @@ int fft_pass(const hx_fft_plan* p, int d, int sign, int batch, int nlines,
     return hx::axis_pass<T>(p->ax[d], sign, batch, nlines, io, scale, min_lines, s);
 }
 
+// Which axis of a 2-D transform goes first.  The two orders run n_src[1] rows and n_dst[0] columns, or n_src[0] columns
+// and n_dst[1] rows; a column pass is the slower one (strided lines, of which a CTA holds two to four, in segments of 16
+// to 32 bytes: 129 us for 4096 columns of 4096 points against 28 us for 1024 rows), so a zero-padded transform takes
+// its few columns first and a cropped one last.
+bool y_first(const hx_fft_plan* p, int direction) {
+    const bool fwd = direction == HX_FORWARD;
+    const int* n_src = fwd ? p->n_in : p->n_out;
+    const int* n_dst = fwd ? p->n_out : p->n_in;
+    const double column = 1.3;  // cost of a strided point to a contiguous one
+    return n_dst[1] * (double)p->N[0] + column * n_src[0] * (double)p->N[1] <
+           n_src[1] * (double)p->N[0] + column * n_dst[0] * (double)p->N[1];
+}
+
 template <typename T>
 int fft_execute_t(const hx_fft_plan* p, int direction, int batch, const void* in, void* out, void* ws,
                   cudaStream_t s) {
@@ -516,10 +531,19 @@ int fft_execute_t(const hx_fft_plan* p, int direction, int batch, const void* in
         return fft_pass<T>(p, 0, sign, 1, batch, in, n_src[0], 1, 0, n_src[0], c_src[0], src_fac(0), out, n_dst[0], 1,
                            0, n_dst[0], c_dst[0], dst_fac(0), scale, 1, s);
     }
-    // pass x: rows of the source (n_src[1] lines) -> intermediate (n_src[1] x n_dst[0])
     const long long src_sz = (long long)n_src[0] * n_src[1];
-    const long long mid_sz = (long long)n_src[1] * n_dst[0];
     const long long dst_sz = (long long)n_dst[0] * n_dst[1];
+    if (y_first(p, direction)) {
+        // pass y: columns of the source (n_src[0] lines, stride n_src[0]) -> intermediate (n_dst[1] x n_src[0])
+        const long long mid_sz = (long long)n_dst[1] * n_src[0];
+        HX_TRY(fft_pass<T>(p, 1, sign, batch, n_src[0], in, 1, n_src[0], src_sz, n_src[1], c_src[1], src_fac(1), ws, 1,
+                           n_src[0], mid_sz, n_dst[1], c_dst[1], dst_fac(1), 1.0, 8, s));
+        // pass x: rows of the intermediate (n_dst[1] lines) -> destination
+        return fft_pass<T>(p, 0, sign, batch, n_dst[1], ws, n_src[0], 1, mid_sz, n_src[0], c_src[0], src_fac(0), out,
+                           n_dst[0], 1, dst_sz, n_dst[0], c_dst[0], dst_fac(0), scale, 1, s);
+    }
+    // pass x: rows of the source (n_src[1] lines) -> intermediate (n_src[1] x n_dst[0])
+    const long long mid_sz = (long long)n_src[1] * n_dst[0];
     HX_TRY(fft_pass<T>(p, 0, sign, batch, n_src[1], in, n_src[0], 1, src_sz, n_src[0], c_src[0], src_fac(0), ws,
                        n_dst[0], 1, mid_sz, n_dst[0], c_dst[0], dst_fac(0), 1.0, 1, s));
     // pass y: columns of the intermediate (n_dst[0] lines, stride n_dst[0]) -> destination
@@ -576,7 +600,8 @@ size_t hx_fft_workspace_bytes(const hx_fft_plan* p, int direction, int batch) {
     const bool fwd = direction == HX_FORWARD;
     const int* n_src = fwd ? p->n_in : p->n_out;
     const int* n_dst = fwd ? p->n_out : p->n_in;
-    return p->esize * (size_t)batch * n_src[1] * n_dst[0];
+    return p->esize * (size_t)batch *
+           (y_first(p, direction) ? (size_t)n_dst[1] * n_src[0] : (size_t)n_src[1] * n_dst[0]);
 }
 
 int hx_fft_execute(const hx_fft_plan* p, int direction, int batch, const void* in, void* out, void* ws,
@@ -661,6 +686,7 @@ int filter_execute_t(const hx_filter_plan* p, int adjoint, int batch, const void
         size_t smem;
         HX_TRY(hx::launch_shape<T>(ax.M, ax.radices, batch, 1, 1, a, &thr, &smem));
         a.tw = (const Cx*)ax.tw.p;
+        a.tws = (const Cx*)ax.tws.p;
         a.n_log = ax.N; a.nlines = batch;
         a.in = (const Cx*)in; a.in_ls = p->n[0]; a.in_es = 1; a.in_bs = 0;
         a.in_count = p->n[0]; a.in_offset = p->c[0]; a.load_add = 0;
@@ -697,6 +723,7 @@ int filter_execute_t(const hx_filter_plan* p, int adjoint, int batch, const void
         size_t smem;
         HX_TRY(hx::launch_shape<T>(ax.M, ax.radices, Nx, batch, 8, a, &thr, &smem));
         a.tw = (const Cx*)ax.tw.p;
+        a.tws = (const Cx*)ax.tws.p;
         a.n_log = Ny; a.nlines = Nx;
         a.in = (const Cx*)ws; a.in_ls = 1; a.in_es = Nx; a.in_bs = w_sz;
         a.in_count = ny; a.in_offset = p->c[1]; a.load_add = 0;

@@ -11,26 +11,93 @@
 // stage with radix R after sub-transforms of length Ns: butterfly j (k = j mod Ns) reads x[j + r N/R], multiplies
 // by W^(r k) with W = exp(-+2 pi i / (Ns R)), and writes (j / Ns) Ns R + k + r Ns.  Shared memory holds one
 // padding element per 16, so the stride-16 writes of the first stage hit distinct banks.
+//
+// CONV (the column pass of the Fourier filter): a forward transform, the product with the transfer function and the
+// inverse transform in one launch.  Thread t holds the spectrum at t + r N/16, which are the inputs of its own first
+// inverse butterfly, so the spectrum never leaves the registers.
+//
+// The kernel is bound by instruction issue (1912 instructions a thread for the 16 points of a 4096-point line in a form
+// with 64-bit index products, general shared-memory indices and a complex scale, 56% issued), so: offsets into shared
+// memory are compile-time constants from one base, every global access is one 32 x 32-bit product from a line pointer,
+// complex additions are packed (two FP32 additions per instruction), and the lines of a CTA synchronise on their own
+// where a line's threads are whole warps.
 #pragma once
 
 #include "fft_line.cuh"
 
 namespace hx {
 
-constexpr int kP2MaxThreads = 512;    // contiguous lines
-constexpr int kP2MaxThreadsLF = 1024; // strided lines
-
 template <int N> struct Pow2Shape {
     static_assert(N == 256 || N == 512 || N == 1024 || N == 2048 || N == 4096, "supported lengths");
     static constexpr int T = N / 16;                  // threads per line
-    static constexpr int S16 = N == 4096 ? 3 : 2;     // radix-16 stages
     static constexpr int RL = N == 4096 ? 1 : N / 256;  // radix of the last stage (1: none)
-    static constexpr int PITCH = N + N / 16;          // shared-memory elements per line
+    // Threads per CTA: 512, two CTAs per SM; 1024 for strided lines of 4096 points, so that a CTA reads and writes
+    // segments of four lines (32 bytes, a sector) and not of two.
+    template <bool LF> __host__ __device__ static constexpr int threads() { return LF && N == 4096 ? 1024 : 512; }
+    // Lines per CTA where there are enough.
+    template <bool LF> __host__ __device__ static constexpr int lines() { return threads<LF>() / T; }
+    // Shared-memory elements per line.  In a column pass a half warp's 16 accesses of 8 bytes are to 16 / lines() points
+    // of lines() lines, which the extra elements spread over the banks.
+    template <bool LF> __host__ __device__ static constexpr int pitch() {
+        return N + N / 16 + (LF ? (lines<LF>() < 16 ? 16 / lines<LF>() : 1) : 0);
+    }
 };
 
-__device__ __forceinline__ int p2idx(int x) { return x + (x >> 4); }
+// ---- packed FP32 ------------------------------------------------------------------------------------------------
 
-// Stage twiddle tables of an N-point line (built at plan time, see p2_stage_tables): for the radix-16 stages
+__device__ __forceinline__ float2 p2_add(float2 a, float2 b) {
+    float2 r;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(r))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return r;
+}
+__device__ __forceinline__ float2 p2_sub(float2 a, float2 b) {
+    // a - b as fma(b, -1, a), which rounds once like the subtraction
+    float2 r;
+    const unsigned long long m1 = 0xbf800000bf800000ull;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(r))
+        : "l"(reinterpret_cast<unsigned long long&>(b)), "l"(m1), "l"(reinterpret_cast<unsigned long long&>(a)));
+    return r;
+}
+
+// 4-point DFT in place over v[i0 + st k] (W = exp(SIGN 2 pi i / 4)).
+template <int SIGN> __device__ __forceinline__ void p2_dft4(float2* v, int i0, int st) {
+    const float2 a = v[i0], b = v[i0 + st], c = v[i0 + 2 * st], d = v[i0 + 3 * st];
+    const float2 t0 = p2_add(a, c), t1 = p2_sub(a, c), t2 = p2_add(b, d), t3 = p2_sub(b, d);
+    v[i0] = p2_add(t0, t2);
+    v[i0 + 2 * st] = p2_sub(t0, t2);
+    if (SIGN < 0) {
+        v[i0 + st] = make_float2(t1.x + t3.y, t1.y - t3.x);
+        v[i0 + 3 * st] = make_float2(t1.x - t3.y, t1.y + t3.x);
+    } else {
+        v[i0 + st] = make_float2(t1.x - t3.y, t1.y + t3.x);
+        v[i0 + 3 * st] = make_float2(t1.x + t3.y, t1.y - t3.x);
+    }
+}
+
+// 16-point DFT as 4 x 4, in slot order: X[k1 + 4 k2] in v[4 k1 + k2] (p2_out).
+template <int SIGN> __device__ __forceinline__ void p2_dft16(float2* v) {
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) p2_dft4<SIGN>(v, n2, 4);
+    v[5] = w16<float, SIGN, 1>(v[5]);
+    v[9] = w16<float, SIGN, 2>(v[9]);
+    v[13] = w16<float, SIGN, 3>(v[13]);
+    v[6] = w16<float, SIGN, 2>(v[6]);
+    v[10] = w16<float, SIGN, 4>(v[10]);
+    v[14] = w16<float, SIGN, 6>(v[14]);
+    v[7] = w16<float, SIGN, 3>(v[7]);
+    v[11] = w16<float, SIGN, 6>(v[11]);
+    v[15] = w16<float, SIGN, 9>(v[15]);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) p2_dft4<SIGN>(v, 4 * k1, 1);
+}
+__host__ __device__ constexpr int p2_out(int r) { return (r >> 2) + 4 * (r & 3); }
+
+// ---- stages -----------------------------------------------------------------------------------------------------
+
+// Stage twiddle tables of an N-point line (built at plan time, see make_stage_tables): for the radix-16 stages
 // NS = 16 and 256, four rows of NS entries, exp(-2 pi i p k / (16 NS)) for p = 1, 2, 4, 8, so that the threads of a
 // warp (consecutive k) read consecutive entries.  Offset of the stage's rows in the table:
 template <int NS> __host__ __device__ constexpr int p2_tw_offset() { return NS == 16 ? 0 : 4 * 16; }
@@ -38,135 +105,179 @@ constexpr int kP2TwEntries = 4 * 16 + 4 * 256;
 
 // v[r] *= W^(r k) for the 16 points of a radix-16 butterfly, W = exp(-+2 pi i / (16 NS)), from the stage's four
 // table rows (W^k, W^2k, W^4k, W^8k) and products at most three deep.
-template <int N, int SIGN, int NS>
+template <int SIGN, int NS>
 __device__ __forceinline__ void p2_twiddle16(float2* v, int k, const float2* __restrict__ tws) {
-    if (k == 0) return;
-    const float2* t = tws + p2_tw_offset<NS>();
-    float2 w1 = __ldg(&t[k]), w2 = __ldg(&t[NS + k]), w4 = __ldg(&t[2 * NS + k]), w8 = __ldg(&t[3 * NS + k]);
+    const float2* t = tws + p2_tw_offset<NS>() + k;
+    float2 w1 = __ldg(t), w2 = __ldg(t + NS), w4 = __ldg(t + 2 * NS), w8 = __ldg(t + 3 * NS);
     if (SIGN > 0) {
         w1.y = -w1.y;
         w2.y = -w2.y;
         w4.y = -w4.y;
         w8.y = -w8.y;
     }
-    const float2 w3 = c_mul(w2, w1);
     float2 wl[8];
     wl[1] = w1;
     wl[2] = w2;
-    wl[3] = w3;
+    wl[3] = c_mul(w2, w1);
     wl[4] = w4;
     wl[5] = c_mul(w4, w1);
     wl[6] = c_mul(w4, w2);
-    wl[7] = c_mul(w4, w3);
-#pragma unroll
-    for (int r = 1; r < 8; ++r) v[r] = c_mul(v[r], wl[r]);
+    wl[7] = c_mul(w4, wl[3]);
     v[8] = c_mul(v[8], w8);
 #pragma unroll
-    for (int r = 1; r < 8; ++r) v[8 + r] = c_mul(v[8 + r], c_mul(w8, wl[r]));
-}
-
-// Radix-16 stage NS (>= 16) read from shared memory: loads, twiddles and the butterfly (result in slot order).
-template <int N, int SIGN, int NS>
-__device__ __forceinline__ void p2_stage16_in(const float2* buf, int t, float2* v, const float2* __restrict__ tws) {
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = buf[p2idx(t + r * (N / 16))];
-    p2_twiddle16<N, SIGN, NS>(v, t & (NS - 1), tws);
-    Dft<float, 16, SIGN>::run(v);
-}
-
-// Writes a radix-16 stage's outputs (slot order) back to shared memory for the next stage.
-template <int SIGN, int NS>
-__device__ __forceinline__ void p2_stage16_out(float2* buf, int t, const float2* v) {
-    const int dst = (t / NS) * 16 * NS + (t & (NS - 1));
-#pragma unroll
-    for (int r = 0; r < 16; ++r) buf[p2idx(dst + Dft<float, 16, SIGN>::out_index(r) * NS)] = v[r];
-}
-
-// grid: x = blocks of lines_per_cta lines, y = batch; blockDim = lines_per_cta * N / 16.  LF: lines adjacent in
-// memory (a column pass), so consecutive threads take consecutive lines and the global accesses coalesce across
-// lines; else consecutive threads take consecutive points of one line.
-template <int N, int SIGN, bool LF>
-__global__ void __launch_bounds__(LF ? kP2MaxThreadsLF : kP2MaxThreads) fft_pow2_kernel(
-    const __grid_constant__ LineArgs<float> a) {
-    using P = Pow2Shape<N>;
-    constexpr int T = P::T;
-    extern __shared__ __align__(16) float2 p2_smem[];
-    const int lpc = a.lines_per_cta;
-    const int ll = LF ? (int)threadIdx.x % lpc : (int)threadIdx.x / T;
-    const int t = LF ? (int)threadIdx.x / lpc : (int)threadIdx.x % T;
-    const long long l = (long long)blockIdx.x * lpc + ll;
-    const bool lok = l < a.nlines;
-    float2* buf = p2_smem + ll * P::PITCH;
-    const float2* in = a.in + a.in_bs * blockIdx.y;
-    float2* out = a.out + a.out_bs * blockIdx.y;
-    const int ladd = ((a.load_add % N) + N) % N;
-    const int soff = ((a.out_offset + a.store_add) % N + N) % N;
-
-    auto store = [&](int kf, float2 val) {
-        int kk = kf - soff;
-        if (kk < 0) kk += N;
-        if (lok && kk < a.out_count) {
-            val = c_mul(val, a.scale);
-            if (a.post) val = c_mul(val, a.post[l * a.post_ls + (long long)kk * a.post_es]);
-            out[l * a.out_ls + (long long)kk * a.out_es] = val;
-        }
-    };
-
-    // ---- stage 0 (radix 16, no twiddles): inputs j = t + r N/16, input p = (j + load_add) mod N - in_offset ----
-    float2 v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        int jj = t + r * T + ladd;
-        if (jj >= N) jj -= N;
-        const int p = jj - a.in_offset;
-        float2 x = make_float2(0.0f, 0.0f);
-        if (lok && p >= 0 && p < a.in_count) {
-            x = in[l * a.in_ls + (long long)p * a.in_es];
-            if (a.pre) x = c_mul(x, a.pre[l * a.pre_ls + p]);
-        }
-        v[r] = x;
+    for (int r = 1; r < 8; ++r) {
+        v[r] = c_mul(v[r], wl[r]);
+        v[8 + r] = c_mul(v[8 + r], c_mul(w8, wl[r]));
     }
-    Dft<float, 16, SIGN>::run(v);
-    p2_stage16_out<SIGN, 1>(buf, t, v);
-    __syncthreads();
+}
 
-    if constexpr (N == 256) {
-        // stage 1 is the last: outputs (t / 16) 256 + t % 16 + m 16 = t + m 16
-        p2_stage16_in<N, SIGN, 16>(buf, t, v, a.tws);
+// Shared-memory element x of a line lies at x + x / 16; the accesses of a stage are one base plus constants.
+// Inputs of butterfly t: x = t + r N/16.
+template <int N> __device__ __forceinline__ void p2_read16(const float2* buf, int t, float2* v) {
+    const float2* p = buf + t + (t >> 4);
 #pragma unroll
-        for (int r = 0; r < 16; ++r) store(t + Dft<float, 16, SIGN>::out_index(r) * 16, v[r]);
-    } else {
-        p2_stage16_in<N, SIGN, 16>(buf, t, v, a.tws);
-        __syncthreads();
-        p2_stage16_out<SIGN, 16>(buf, t, v);
-        __syncthreads();
+    for (int r = 0; r < 16; ++r) v[r] = p[r * (N / 16 + N / 256)];
+}
+// Outputs of stage NS = 1 (x = 16 t + m) and NS = 16 (x = 256 (t / 16) + t % 16 + 16 m), from slot order.
+template <int NS> __device__ __forceinline__ void p2_write16(float2* buf, int t, const float2* v) {
+    float2* p = NS == 1 ? buf + 17 * t : buf + 272 * (t >> 4) + (t & 15);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) p[p2_out(r) * (NS == 1 ? 1 : 17)] = v[r];
+}
+
+// The lines of a CTA in step: a line's threads alone where they are whole warps of one line.
+template <int T, bool LF> __device__ __forceinline__ void p2_sync(int line) {
+    if constexpr (LF) __syncthreads();
+    else if constexpr (T == 32) __syncwarp();
+    else if constexpr (T >= 64) asm volatile("bar.sync %0, %1;" ::"r"(line + 1), "r"(T) : "memory");
+    else __syncthreads();
+}
+
+// Transform of the 16 values v[r] = x[t + r N/16] of a line; on return v[p2_slot<N>(s)] = X[t + s N/16].
+template <int N, int SIGN, bool LF>
+__device__ __forceinline__ void p2_transform(float2* v, float2* buf, int t, int line, const float2* __restrict__ tw,
+                                             const float2* __restrict__ tws) {
+    constexpr int T = N / 16;
+    p2_dft16<SIGN>(v);
+    p2_write16<1>(buf, t, v);
+    p2_sync<T, LF>(line);
+    p2_read16<N>(buf, t, v);
+    p2_twiddle16<SIGN, 16>(v, t & 15, tws);
+    p2_dft16<SIGN>(v);
+    if constexpr (N > 256) {
+        p2_sync<T, LF>(line);
+        p2_write16<16>(buf, t, v);
+        p2_sync<T, LF>(line);
         if constexpr (N == 4096) {
-            // stage 2 is the last: outputs t + m 256
-            p2_stage16_in<N, SIGN, 256>(buf, t, v, a.tws);
-#pragma unroll
-            for (int r = 0; r < 16; ++r) store(t + Dft<float, 16, SIGN>::out_index(r) * 256, v[r]);
+            p2_read16<N>(buf, t, v);
+            p2_twiddle16<SIGN, 256>(v, t, tws);
+            p2_dft16<SIGN>(v);
         } else {
-            // last stage, radix RL after 256-point sub-transforms: butterflies b = t + i N/16 (i < 16 / RL), inputs
-            // b + r 256, twiddles W_N^(r b), outputs b + r 256 in natural order
-            constexpr int RL = P::RL;
+            // last stage, radix RL after 256-point sub-transforms: butterflies b = t + i T (i < 16 / RL), inputs
+            // b + 256 r, twiddles W_N^(r b), outputs b + 256 r = t + (i + 16 / RL r) T
+            constexpr int RL = Pow2Shape<N>::RL, NB = 16 / RL;
+            const float2* p = buf + t + (t >> 4);
 #pragma unroll
-            for (int i = 0; i < 16 / RL; ++i) {
-                const int b = t + i * T;
+            for (int i = 0; i < NB; ++i) {
                 float2 u[RL];
 #pragma unroll
                 for (int r = 0; r < RL; ++r) {
-                    u[r] = buf[p2idx(b + r * 256)];
+                    // element t + i T + 256 r: t / 16 carries into the padding only with T a multiple of 16
+                    u[r] = p[(i * T + 256 * r) + ((i * T + 256 * r) >> 4)];
                     if (r > 0) {
-                        float2 w = a.tw[r * b];
+                        float2 w = __ldg(&tw[r * (t + i * T)]);
                         if (SIGN > 0) w.y = -w.y;
                         u[r] = c_mul(u[r], w);
                     }
                 }
                 Dft<float, RL, SIGN>::run(u);
 #pragma unroll
-                for (int r = 0; r < RL; ++r) store(b + r * 256, u[r]);
+                for (int r = 0; r < RL; ++r) v[i + NB * r] = u[r];
             }
         }
+    }
+}
+// Register of X[t + s N/16] after p2_transform.
+template <int N> __host__ __device__ constexpr int p2_slot(int s) {
+    return (N == 256 || N == 4096) ? p2_out(s) : s;  // p2_out is its own inverse
+}
+
+// grid: x = blocks of lines_per_cta lines, y = batch; blockDim = lines_per_cta * N / 16.  LF: lines adjacent in
+// memory (a column pass), so consecutive threads take consecutive lines and the global accesses coalesce across
+// lines; else consecutive threads take consecutive points of one line.  CONV: SIGN is that of the first transform.
+template <int N, int SIGN, bool LF, bool CONV>
+__global__ void __launch_bounds__(Pow2Shape<N>::template threads<LF>(), 1024 / Pow2Shape<N>::template threads<LF>())
+    fft_pow2_kernel(const __grid_constant__ LineArgs<float> a) {
+    constexpr int T = Pow2Shape<N>::T;
+    extern __shared__ __align__(16) float2 p2_smem[];
+    const int lpc = a.lines_per_cta;
+    const int line = LF ? (int)threadIdx.x & (lpc - 1) : (int)threadIdx.x / T;
+    const int t = LF ? (int)threadIdx.x >> (31 - __clz(lpc)) : (int)threadIdx.x % T;
+    const long long l = (long long)blockIdx.x * lpc + line;
+    const bool lok = l < a.nlines;
+    float2* buf = p2_smem + line * Pow2Shape<N>::template pitch<LF>();
+    const float2* in = a.in + a.in_bs * blockIdx.y + l * a.in_ls;
+    float2* out = a.out + a.out_bs * blockIdx.y + l * a.out_ls;
+    const int in_es = LF ? (int)a.in_es : 1, out_es = LF ? (int)a.out_es : 1;
+
+    // ---- inputs x[t + r T], taken from position (t + r T + load_add - in_offset) mod N of the input line -----------
+    const int lshift = (a.load_add - a.in_offset) & (N - 1);
+    float2 v[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const int p = (t + r * T + lshift) & (N - 1);
+        v[r] = make_float2(0.0f, 0.0f);
+        if (lok && p < a.in_count) v[r] = in[(long long)p * in_es];
+    }
+    if (a.pre) {
+        const float2* pre = a.pre + l * a.pre_ls;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const int p = (t + r * T + lshift) & (N - 1);
+            if (lok && p < a.in_count) v[r] = c_mul(v[r], pre[p]);
+        }
+    }
+    p2_transform<N, SIGN, LF>(v, buf, t, line, a.tw, a.tws);
+    if constexpr (CONV) {
+        const int mid_es = (int)a.mid_es;
+        const float2* mid = a.mid + l * a.mid_ls + (long long)t * mid_es;
+        const float cs = a.mid_conj ? -1.0f : 1.0f;
+        float2 u[16];
+#pragma unroll
+        for (int s = 0; s < 16; ++s) {
+            float2 m = make_float2(0.0f, 0.0f);
+            if (lok) m = __ldg(mid + (long long)(s * T) * mid_es);
+            m.y *= cs;
+            u[s] = c_mul(v[p2_slot<N>(s)], m);
+        }
+        p2_sync<T, LF>(line);  // the last reads of the first transform
+        p2_transform<N, -SIGN, LF>(u, buf, t, line, a.tw, a.tws);
+#pragma unroll
+        for (int s = 0; s < 16; ++s) v[s] = u[s];
+    }
+
+    // ---- output (t + s T - out_offset - store_add) mod N of the output line is X[t + s T] ---------------------------
+    const int sshift = (-(a.out_offset + a.store_add)) & (N - 1);
+    if (a.scale.y != 0.0f) {
+#pragma unroll
+        for (int s = 0; s < 16; ++s) v[s] = c_mul(v[s], a.scale);
+    } else if (a.scale.x != 1.0f) {
+#pragma unroll
+        for (int s = 0; s < 16; ++s) v[s] = make_float2(v[s].x * a.scale.x, v[s].y * a.scale.x);
+    }
+    if (a.post) {
+        const float2* post = a.post + l * a.post_ls;
+        const int post_es = (int)a.post_es;
+#pragma unroll
+        for (int s = 0; s < 16; ++s) {
+            const int kk = (t + s * T + sshift) & (N - 1);
+            if (lok && kk < a.out_count) v[p2_slot<N>(s)] = c_mul(v[p2_slot<N>(s)], post[(long long)kk * post_es]);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < 16; ++s) {
+        const int kk = (t + s * T + sshift) & (N - 1);
+        if (lok && kk < a.out_count) out[(long long)kk * out_es] = v[p2_slot<N>(s)];
     }
 }
 
