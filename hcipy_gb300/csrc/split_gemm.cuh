@@ -42,7 +42,7 @@
 // warp 0 issues TMA loads (one 3-D box per operand per stage:
 // three slice planes of 64 K-elements, 128-byte swizzle), warp 1 issues
 // tcgen05.mma (8 slice products x 4 K16 steps per stage) into four TMEM
-// accumulators of 128 lanes x BN columns, warps 2-9 read TMEM, combine and
+// accumulators of 128 lanes x BN columns, warps 2-17 read TMEM, combine and
 // finish the result.  Three stages of 72 KiB (BN = 64) or two of 96 KiB
 // (BN = 128).  GEMMs with too few tiles to fill the GPU split K across CTAs:
 // each CTA combines its levels into a float-float partial (level 0 exactly),
@@ -75,7 +75,12 @@ constexpr int BK = 64;   // K' elements per stage (128 bytes of fp16)
 constexpr int NSLICE = 3;
 constexpr int A_PLANE_BYTES = BM * BK * 2;
 constexpr int A_STAGE_BYTES = NSLICE * A_PLANE_BYTES;
-constexpr int NUM_THREADS = 320;  // TMA warp, MMA warp, 8 epilogue warps
+// Epilogue warps, four per TMEM lane quarter.  One CTA fills an SM, so while it finishes its tile nothing else runs
+// there, and what bounds the epilogue is its own latencies (TMEM reads, chains of float-float steps, the stores).
+// Sixteen warps instead of eight: a complex128 Lyot pass over 2048^2 points 562 -> 549 us, a gradient step over 64
+// fields of 512^2 points 6471 -> 6035 us (most tiles, each with few K steps), the same bits.
+constexpr int EPI_WARPS = 16;
+constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;  // TMA warp, MMA warp, epilogue warps
 constexpr uint64_t WAIT_LIMIT = 2000000000ull;  // 2 s per wait
 constexpr int MAX_SPLIT_K = 4096;               // exact level-0 sums need at most 4096 K' per CTA
 constexpr int MAX_SPLIT_KTILES = MAX_SPLIT_K / BK;
@@ -457,12 +462,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_accum, 0, WAIT_LIMIT)) && ok;
         if (!ok && leader) raise_status(g.status, abort_flag);
     }
-    // ---- epilogue: warps 2..9, two per TMEM lane quarter (each takes every other 16-column chunk) ----------
+    // ---- epilogue: warps 2..17, four per TMEM lane quarter (each takes every fourth 16-column chunk) --------
     constexpr int EPI = NUM_THREADS - 64;
     const bool epi_warp = warp >= 2;
     const int et = threadIdx.x - 64;         // 0..EPI-1 on the epilogue warps
     const int quarter = warp & 3;            // TMEM lane quarter this warp may access
-    const int half = (warp - 2) >> 2;        // 0 or 1
+    const int slot = (warp - 2) >> 2;        // this warp's among those of its quarter
+    constexpr int SLOTS = EPI_WARPS / 4;
     const int row = quarter * 32 + lane;     // A' row within the tile = TMEM lane
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     bool live = false;
@@ -473,13 +479,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         live = __shfl_sync(0xffffffffu, (int)(*abort_flag == 0), 0) != 0;
     }
     auto own_chunk = [&](int c, ff* r) {
-        float v0[16], v1[16], v2[16], v3[16];
-        ptx::tmem_ld_16(tmem + lane_base + 0 * BN + c * 16, v0);
-        ptx::tmem_ld_16(tmem + lane_base + 1 * BN + c * 16, v1);
-        ptx::tmem_ld_16(tmem + lane_base + 2 * BN + c * 16, v2);
-        ptx::tmem_ld_16(tmem + lane_base + 3 * BN + c * 16, v3);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = combine_levels(v0[j], v1[j], v2[j], v3[j]);
+        for (int h = 0; h < 16; h += 8) {  // 8 columns of the four levels at a time (registers)
+            float v0[8], v1[8], v2[8], v3[8];
+            const uint32_t at = tmem + lane_base + c * 16 + h;
+            ptx::tmem_ld_8x4(at, BN, v0, v1, v2, v3);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[h + j] = combine_levels(v0[j], v1[j], v2[j], v3[j]);
+        }
     };
     // The slice of the tile this CTA finishes: all of it, or with a cluster of S splits the q-th of S column
     // slices (W = BN / S TMEM columns, TNs complex columns; W is a multiple of 16, so with EMB = 1 a slice holds
@@ -504,7 +511,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         ptx::cluster_sync();  // every CTA's copies and MMAs are complete: its pipeline buffers are free
         if (epi_warp && live) {
 #pragma unroll 1
-            for (int c = half; c < BN / 16; c += 2) {
+            for (int c = slot; c < BN / 16; c += SLOTS) {
                 ff r[16];
                 own_chunk(c, r);
                 const int dst = (c * 16) / W;
@@ -562,7 +569,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         if (g.ksplit > 1) {
             if (live) {
 #pragma unroll 1
-                for (int c = half; c < BN / 16; c += 2) {
+                for (int c = slot; c < BN / 16; c += SLOTS) {
                     ff r[16];
                     own_chunk(c, r);
 #pragma unroll
@@ -580,7 +587,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
             if (finish && live) {
                 __threadfence();
 #pragma unroll 1
-                for (int c = half; c < BN / 16; c += 2) {
+                for (int c = slot; c < BN / 16; c += SLOTS) {
                     ff own[16], acc[16];
                     own_chunk(c, own);
                     // Splits in index order (the sum does not depend on which CTA finishes last); two at a time.
@@ -624,7 +631,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
             }
         } else if (live) {
 #pragma unroll 1
-            for (int c = half; c < BN / 16; c += 2) {
+            for (int c = slot; c < BN / 16; c += SLOTS) {
                 ff r[16];
                 own_chunk(c, r);
 #pragma unroll
@@ -658,14 +665,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
             const int c_re = EMB ? (nl >> 3) * 16 + (nl & 7) : nl;
             const int c_im = EMB ? c_re + 8 : nl;
             constexpr int R_IM = EMB ? 0 : 64;
-            const int RSTEP = EPI / TNS;          // rows per iteration
-            const int ITER = TM / RSTEP;          // a multiple of U for every tile and slice width in use
+            // rows per iteration: a power of two, so that whole iterations make up the tile's rows
+            const int RSTEP = min(TM, 1 << (31 - __clz(EPI / TNS)));
+            const int ITER = TM / RSTEP;
             constexpr int U = 4;                  // rows per batch: loads issued before any store
-            // With TNs not dividing the epilogue threads (BN = 112) the last EPI - RSTEP * TNs threads have no
-            // column; they skip the loop so that no row beyond the tile's TM is touched.
+            // Threads past RSTEP * TNs (BN = 112) have no column; they skip the loop so that no row beyond the tile's
+            // TM is touched.
             const bool has_col = et < RSTEP * TNS;
             const int r0 = et / TNS;
-            const int mlim = g.M - m_tile * TM;   // valid rows of this tile
+            const int mlim = min(TM, g.M - m_tile * TM);  // valid rows of this tile
             int cfield = -1;
             float cmax = 0.0f;
 #pragma unroll 1
@@ -715,7 +723,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                     if (g.rowmax) {
                         if (EMB) {
                             if (mag > 0.0f) atomicMax(&s_rowmax[ml], __float_as_uint(mag));
-                        } else {
+                        } else if (ml < TM) {
                             s_mag[ml * fpitch + nl] = mag;
                         }
                     }

@@ -133,6 +133,23 @@ __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 8 consecutive columns of four accumulators `step` columns apart.
+__device__ __forceinline__ void tmem_ld_8x4(uint32_t taddr, uint32_t step, float* a, float* b, float* c, float* d) {
+    float* out[4] = {a, b, c, d};
+    uint32_t r[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[i][0]), "=r"(r[i][1]), "=r"(r[i][2]), "=r"(r[i][3]), "=r"(r[i][4]), "=r"(r[i][5]),
+                       "=r"(r[i][6]), "=r"(r[i][7])
+                     : "r"(taddr + i * step));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) out[i][j] = __uint_as_float(r[i][j]);
+}
+
 // ---- thread-block clusters -------------------------------------------------------------------------
 
 // Every thread of every CTA of the cluster arrives (release) and waits (acquire): shared-memory writes made
