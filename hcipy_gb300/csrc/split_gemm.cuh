@@ -41,7 +41,7 @@
 // tile of B' (EMB = 0; with EMB = 1, 128 complex rows x BN/2 complex columns).
 // warp 0 issues TMA loads (one 3-D box per operand per stage:
 // three slice planes of 64 K-elements, 128-byte swizzle), warp 1 issues
-// tcgen05.mma (8 slice products x 4 K16 steps per stage) into four TMEM
+// tcgen05.mma (8 slice products x 4 K16 steps per stage, several per MMA) into four TMEM
 // accumulators of 128 lanes x BN columns, warps 2-17 read TMEM, combine and
 // finish the result.  Three stages of 72 KiB (BN = 64) or two of 96 KiB
 // (BN = 128).  GEMMs with too few tiles to fill the GPU split K across CTAs:
@@ -425,16 +425,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         // The whole warp runs this branch with only the instructions themselves under the elected lane: issued from a
         // one-lane branch, with 64-bit descriptors built for each, an MMA took 79 clocks of the issuing thread where
         // the 128-column product itself takes 64.
-        constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN);
         // descriptors of a K-major operand with 128-byte swizzle: 8-row groups 1024 B apart, version 1, swizzle mode 2
         constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
         const bool leader = ptx::elect_one();
-        // (A slice, B slice, level) of the kept products; the first product of a level starts it.
-        constexpr int NPROD = 8;
-        const int pa[NPROD] = {0, 0, 1, 0, 1, 2, 1, 2};
-        const int pb[NPROD] = {0, 1, 0, 2, 1, 0, 2, 1};
-        const int pl[NPROD] = {0, 1, 1, 2, 2, 2, 3, 3};
-        const int first[NPROD] = {1, 1, 0, 1, 0, 0, 1, 0};
+        // The kept products are a0 (b0 b1 b2), a1 (b0 b1 b2), a2 (b0 b1), the levels being the sums of the indices.  The
+        // slices of B follow one another in shared memory as the levels do in TMEM, so one MMA multiplies a slice of
+        // A by several of B: as many as 256 columns hold.  What bounds the loop is shared memory, and each MMA reads its
+        // A again (4 KB): with 128 columns 5 MMAs and 52 KB per 16 K' instead of 8 and 64 KB, with 64 columns 3 and
+        // 28 KB instead of 8 and 48 KB (512 x 512 outputs over 2048 points with 64 columns: 48 -> 39 us; a Lyot pass
+        // over 2048^2 points 549 -> 527 us, the same bits; a stage with 128 columns now takes 2220 clocks, its MMAs
+        // 2048).  The order of the products within a level is that of the single ones.
+        constexpr int MAXS = 256 / BN < NSLICE ? 256 / BN : NSLICE;  // slices of B per MMA
         bool ok = true;
         for (int i = 0; i < nkt; ++i) {
             const int s = i % STAGES;
@@ -444,15 +445,27 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
             ptx::tc_fence_after();
             const uint32_t a0 = (((smem_base + s * T::STAGE_BYTES) & 0x3FFFF) >> 4) | (1u << 16);
             const uint32_t b0 = a0 + (A_STAGE_BYTES >> 4);
+            auto mma = [&](auto count, int pa, int pb, int kk, bool start) {
+                constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN * decltype(count)::value);
+                if (leader)
+                    ptx::umma_f16_lo(tmem + (pa + pb) * BN, a0 + ((pa * A_PLANE_BYTES + kk * 32) >> 4),
+                                     b0 + ((pb * T::B_PLANE_BYTES + kk * 32) >> 4), desc_hi, idesc, start);
+            };
+            using one = std::integral_constant<int, 1>;
+            using two = std::integral_constant<int, 2>;
+            using most = std::integral_constant<int, MAXS>;
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk) {
-#pragma unroll
-                for (int p = 0; p < NPROD; ++p) {
-                    if (leader)
-                        ptx::umma_f16_lo(tmem + pl[p] * BN, a0 + ((pa[p] * A_PLANE_BYTES + kk * 32) >> 4),
-                                         b0 + ((pb[p] * T::B_PLANE_BYTES + kk * 32) >> 4), desc_hi, idesc,
-                                         i == 0 && kk == 0 && first[p]);
+                const bool start = i == 0 && kk == 0;  // the first product of a level starts it
+                mma(most{}, 0, 0, kk, start);
+                if (MAXS < 3) mma(one{}, 0, 2, kk, start);
+                if (MAXS < 3 || start) {  // a1 b2 starts level 3
+                    mma(two{}, 1, 0, kk, false);
+                    mma(one{}, 1, 2, kk, start);
+                } else {
+                    mma(most{}, 1, 0, kk, false);
                 }
+                mma(two{}, 2, 0, kk, false);
             }
             if (leader) ptx::umma_commit(bar_empty(s));
         }
