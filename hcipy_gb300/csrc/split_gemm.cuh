@@ -205,11 +205,27 @@ __device__ __forceinline__ unsigned long long float_bits_to_double_bits(unsigned
     return sign | ((unsigned long long)(e + 896) << 52) | ((unsigned long long)m << 29);
 }
 
-// hi + lo as float64: each float is placed exactly into float64 bits (integer operations), then one float64
-// addition rounds the sum.
+// hi + lo as float64, rounded to nearest even.  The float64 pipe takes about 1.6 operations a clock and SM, so the sum is
+// made with integers: hi's bits placed as a float64 leave 29 zeros below, to which lo is added as a whole number of ulps
+// (lo scaled by a power of two and rounded to an int; |lo| <= ulp(hi) / 2 is 2^28 of them at most, which reaches neither
+// the exponent from below nor, with a fraction of hi that is not zero, from above).  hi below 2^-75 or beyond the floats,
+// a power of two less a lo, and pairs that are not normalised take the float64 addition; both ways give the same bits.
 __device__ __forceinline__ double ff_to_double(ff v) {
-    return __dadd_rn(__longlong_as_double((long long)float_bits_to_double_bits(__float_as_uint(v.hi))),
-                     __longlong_as_double((long long)float_bits_to_double_bits(__float_as_uint(v.lo))));
+    const unsigned int h = __float_as_uint(v.hi), l = __float_as_uint(v.lo);
+    if (((h | l) << 1) == 0) return __hiloint2double((int)(h & l), 0);
+    const unsigned int e = (h >> 23) & 0xff;
+    if (e >= 52 && e < 255 && ((h & 0x7fffffu) != 0 || ((h ^ l) & 0x80000000u) == 0)) {
+        const float ulps = v.lo * __uint_as_float((306 - e) << 23);
+        if (fabsf(ulps) <= 0x1p28f) {
+            int k = __float2int_rn(ulps);
+            if (h & 0x80000000u) k = -k;
+            const unsigned int up = (h & 0x80000000u) | (((h & 0x7fffffffu) >> 3) + (896u << 20));
+            const long long bits = (long long)(((unsigned long long)up << 32) | (h << 29)) + k;
+            return __longlong_as_double(bits);
+        }
+    }
+    return __dadd_rn(__longlong_as_double((long long)float_bits_to_double_bits(h)),
+                     __longlong_as_double((long long)float_bits_to_double_bits(l)));
 }
 
 template <int FMT> __device__ __forceinline__ cff load_fmt(const FieldIO& f, long long i) {
@@ -734,7 +750,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                         }
                     }
                     if (g.rowmax) {
-                        if (EMB) {
+                        if (EMB && TNC > 0 && TNC % 32 == 0) {  // a warp holds columns of one row
+                            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mag));
+                            if (lane == 0 && m > 0) atomicMax(&s_rowmax[ml], m);
+                        } else if (EMB) {
                             if (mag > 0.0f) atomicMax(&s_rowmax[ml], __float_as_uint(mag));
                         } else if (ml < TM) {
                             s_mag[ml * fpitch + nl] = mag;
