@@ -60,20 +60,31 @@ def von_karman_covariance(r, r0, L0):  # noqa: N803
     return a * b * c * d * e
 
 
+_QUINTIC = (1.0, -6.0, 15.0, -20.0, 15.0, -6.0, 1.0)
+
+
+def _quintic_taps(shift):
+    """``quintic_weights`` as a list."""
+    shift = float(shift)
+    f = abs(shift)
+    b = []
+    for offset in (2.0 + f, 1.0 + f, f, 1.0 - f, 2.0 - f, 3.0 - f):
+        acc, x = 0.0, offset + 3.0
+        for c in _QUINTIC:
+            if x <= 0.0:  # x only falls: the terms that follow are zero
+                break
+            acc += c * x**5
+            x -= 1.0
+        b.append(acc / 120.0)
+    if shift >= 0:
+        return [0.0] + b
+    b.reverse()
+    return b + [0.0]
+
+
 def quintic_weights(shift):
     """7-tap quintic B-spline weights of a shift in [-0.5, 0.5] pixels (subpixel_shift.py:7-35)."""
-    f = abs(shift)
-    b = np.empty(6)
-    for i, offset in enumerate((2.0 + f, 1.0 + f, f, 1.0 - f, 2.0 - f, 3.0 - f)):
-        acc, x = 0.0, offset + 3.0
-        for c in (1.0, -6.0, 15.0, -20.0, 15.0, -6.0, 1.0):
-            if x > 0.0:
-                acc += c * x**5
-            x -= 1.0
-        b[i] = acc / 120.0
-    if shift >= 0:
-        return np.array([0.0, b[0], b[1], b[2], b[3], b[4], b[5]])
-    return np.array([b[5], b[4], b[3], b[2], b[1], b[0], 0.0])
+    return np.array(_quintic_taps(shift))
 
 
 def power_spectral_density_von_karman(r0, L0):  # noqa: N803
@@ -234,11 +245,9 @@ def subpixel_shift(img, row_shift, col_shift):
         t = t.to(torch.float64)
     ny, nx = t.shape[-2:]
     out = torch.empty_like(t)
-    tr = np.ascontiguousarray(quintic_weights(col_shift))
-    tc = np.ascontiguousarray(quintic_weights(row_shift))
-    P = _lib.ctypes.POINTER(_lib.ctypes.c_double)
-    rc = _lib.lib().hx_atmosphere_shift(_lib.dptr(t), int(ny), int(nx), int(ny), int(nx), 0, 0, tr.ctypes.data_as(P),
-                                        tc.ctypes.data_as(P), _lib.dptr(out), _lib.dtype_code(t.dtype),
+    taps = _lib.c_double * 7
+    rc = _lib.lib().hx_atmosphere_shift(_lib.dptr(t), ny, nx, ny, nx, 0, 0, taps(*_quintic_taps(col_shift)),
+                                        taps(*_quintic_taps(row_shift)), _lib.dptr(out), _lib.dtype_code(t.dtype),
                                         _lib.stream_handle())
     _lib.check(rc, 'hx_atmosphere_shift')
     return out

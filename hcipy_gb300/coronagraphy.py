@@ -1,6 +1,7 @@
 """Coronagraphs: the Lyot coronagraph (hcipy/coronagraphy/lyot.py:7-122) with the Babinet chain fused into the MFT
 GEMMs, and the multi-scale, vortex and vector-vortex coronagraphs (multi_scale.py, vortex.py)."""
 import collections
+import math
 
 import numpy as np
 import torch
@@ -94,7 +95,7 @@ class LyotCoronagraph(OpticalElement):
         ft = inst.fourier_transform
         t = t.detach().contiguous()
         lead = tuple(t.shape[:-1])
-        batch = int(np.prod(lead)) if lead else 1
+        batch = math.prod(lead)
         out = torch.empty(lead + (t.shape[-1],), dtype=out_dtype, device=t.device)
         if batch == 0:
             return out
@@ -146,7 +147,6 @@ class MultiScaleCoronagraph(OpticalElement):
         from scipy.signal import windows
         from .fft import FastFourierTransform, FourierFilter
         from .field import make_focal_grid
-        import math
         self.input_grid = input_grid
         pupil_diameter = np.asarray(input_grid.dims, np.float64) * np.asarray(input_grid.delta, np.float64)
         if hasattr(lyot_stop, 'forward') or lyot_stop is None:

@@ -128,7 +128,7 @@ class FastFourierTransform(FourierTransform):
     def _run(self, field, src_grid, dst_grid, direction):
         t = _prepare_input(field, src_grid)
         batch_shape = tuple(t.shape[:-1])
-        batch = int(np.prod(batch_shape)) if batch_shape else 1
+        batch = math.prod(batch_shape)
         out = torch.empty(batch_shape + (dst_grid.size,), dtype=t.dtype, device=t.device)
         if batch > 0:
             lib = _lib.lib()
@@ -227,7 +227,7 @@ class ChirpZTransform(object):
         if t.shape[-1] != self.n:
             raise ValueError('The last axis must have %d points.' % self.n)
         lead = tuple(t.shape[:-1])
-        lines = int(np.prod(lead)) if lead else 1
+        lines = math.prod(lead)
         out = torch.empty(lead + (self.m,), dtype=cdt, device=t.device)
         if lines:
             plan = self._plan(cdt)
@@ -286,7 +286,7 @@ class ZoomFastFourierTransform(FourierTransform):
     def _run(self, field, src, dst, inverse):
         t = _prepare_input(field, src)
         lead = tuple(t.shape[:-1])
-        batch = int(np.prod(lead)) if lead else 1
+        batch = math.prod(lead)
         out = torch.empty(lead + (dst.size,), dtype=t.dtype, device=t.device)
         if batch == 0:
             return Field(out, dst)
@@ -437,7 +437,7 @@ class FourierFilter(object):
     def _operation(self, field, adjoint):
         t = _prepare_input(field, self.input_grid)
         lead = tuple(t.shape[:-1])
-        batch = int(np.prod(lead)) if lead else 1
+        batch = math.prod(lead)
         out = torch.empty_like(t)
         if batch:
             lib = _lib.lib()

@@ -46,7 +46,7 @@ class RegularCoords(object):
 
     @property
     def size(self):
-        return int(np.prod(self.dims))
+        return math.prod(self.dims.tolist())
 
     @property
     def separated_coords(self):
@@ -86,7 +86,7 @@ class SeparatedCoords(object):
 
     @property
     def size(self):
-        return int(np.prod(self.dims))
+        return math.prod(int(d) for d in self.dims)
 
     def scaled(self, s):
         s = np.broadcast_to(np.asarray(s, np.float64), (self.ndim,))
@@ -431,9 +431,9 @@ def as_tensor(x, device='cuda'):
     else:
         arr = np.asarray(x)
         t = torch.from_numpy(np.ascontiguousarray(arr))
-    if t.device.type != 'cuda':
+    if not t.is_cuda:
         t = t.to(device, non_blocking=False)
-    if t.is_complex() and t.is_conj():  # a lazy conjugate view: the kernels read memory, so materialise it
+    if t.is_conj():  # a lazy conjugate view: the kernels read memory, so materialise it
         t = t.resolve_conj()
     return t
 
@@ -451,7 +451,7 @@ class Field(object):
             if grid is None:
                 grid = data.grid
             data = data.data
-        self.data = as_tensor(data)
+        self.data = data if type(data) is torch.Tensor and data.is_cuda and not data.is_conj() else as_tensor(data)
         self.grid = grid
 
     def __reduce__(self):

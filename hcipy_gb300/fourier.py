@@ -274,7 +274,7 @@ class MatrixFourierTransform(FourierTransform):
              out=None):
         t = _prepare_input(field, src_grid)
         batch_shape = tuple(t.shape[:-1])
-        batch = int(np.prod(batch_shape)) if batch_shape else 1
+        batch = math.prod(batch_shape)
         split = self.precision == 'split'
         if out is None:
             out_dtype = torch.complex128 if split else t.dtype

@@ -2,6 +2,8 @@
 
 Every function launches a kernel of ``lib/libhcipy_gb300.so``; there is no CPU path.
 """
+import math
+
 import numpy as np
 import torch
 
@@ -26,17 +28,24 @@ def apply_phase(e, s, scale):
     """
     n = e.shape[-1]
     rdt = _REAL[e.dtype]
-    s = s.to(device=e.device, dtype=rdt)
+    if s.dtype != rdt or s.device != e.device:
+        s = s.to(device=e.device, dtype=rdt)
     shape_e, shape_s = tuple(e.shape[:-1]), tuple(s.shape[:-1])
-    be = int(np.prod(shape_e)) if shape_e else 1
-    bs = int(np.prod(shape_s)) if shape_s else 1
+    be, bs = math.prod(shape_e), math.prod(shape_s)
     batch = max(be, bs) if be and bs else 0  # an empty batch on either side gives an empty result
-    try:
-        lead = tuple(torch.broadcast_shapes(shape_e, shape_s))  # keeps a batch of one given on either side
-    except RuntimeError:
-        lead = shape_e if be >= bs else shape_s
-    out_shape = (lead if int(np.prod(lead)) == batch else (shape_e if be >= bs else shape_s)) + (n,)
-    e2, s2 = _batched(e, n), _batched(s, n)
+    if shape_e == shape_s or not shape_s:
+        lead = shape_e
+    elif not shape_e:
+        lead = shape_s
+    else:
+        try:
+            lead = tuple(torch.broadcast_shapes(shape_e, shape_s))  # keeps a batch of one given on either side
+        except RuntimeError:
+            lead = shape_e if be >= bs else shape_s
+    out_shape = (lead if math.prod(lead) == batch else (shape_e if be >= bs else shape_s)) + (n,)
+    if s.shape[-1] != n:
+        raise ValueError('expected a last axis of %d elements, got %s' % (n, tuple(s.shape)))
+    e2, s2 = e.contiguous(), s.contiguous()
     out = torch.empty(out_shape, dtype=e.dtype, device=e.device)
     if out.numel() == 0:
         return out
@@ -52,8 +61,7 @@ def apply_phase_grad(e, s, scale, g_out, need_e=True, need_s=True):
     rdt = _REAL[e.dtype]
     s = s.to(device=e.device, dtype=rdt)
     shape_e, shape_s = tuple(e.shape[:-1]), tuple(s.shape[:-1])
-    be = int(np.prod(shape_e)) if shape_e else 1
-    bs = int(np.prod(shape_s)) if shape_s else 1
+    be, bs = math.prod(shape_e), math.prod(shape_s)
     batch = max(be, bs) if be and bs else 0  # an empty batch on either side gives an empty result
     e2, s2 = _batched(e, n), _batched(s, n)
     g2 = _batched(g_out.to(e.dtype), n)
@@ -165,7 +173,7 @@ def intensity_sums(e, w=None):
         raise TypeError('intensity sums take complex64 or complex128 fields, not %s' % e.dtype)
     n = e.shape[-1]
     lead = tuple(e.shape[:-1])
-    batch = int(np.prod(lead)) if lead else 1
+    batch = math.prod(lead)
     out = torch.zeros(lead, dtype=torch.float64, device=e.device)
     if batch == 0 or n == 0:
         return out
@@ -185,7 +193,7 @@ def intensity_sums_grad(e, w, g):
     """Gradient of ``intensity_sums`` in torch's convention: 2 g[b] w e_b, in e's dtype and shape."""
     n = e.shape[-1]
     lead = tuple(e.shape[:-1])
-    batch = int(np.prod(lead)) if lead else 1
+    batch = math.prod(lead)
     out = torch.empty(lead + (n,), dtype=e.dtype, device=e.device)
     if batch == 0 or n == 0:
         return out

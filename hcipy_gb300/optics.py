@@ -255,9 +255,12 @@ class InstanceData(object):
         self.wavelength = wavelength
 
 
+_LOG_STEP = math.log(1 + 1e-9)
+
+
 def _wavelength_key(wavelength):
     # hcipy/optics/optical_element.py:333.
-    return int(np.round(np.log(wavelength) / np.log(1 + 1e-9)))
+    return round(math.log(wavelength) / _LOG_STEP)
 
 
 class AgnosticOpticalElement(OpticalElement):

@@ -1,4 +1,6 @@
 """Propagators (hcipy/propagation) on the device."""
+import math
+
 import numpy as np
 import torch
 
@@ -107,7 +109,7 @@ class FraunhoferPropagator(AgnosticOpticalElement):
         ft = inst.fourier_transform
         t = t.contiguous()
         lead = tuple(t.shape[:-1])
-        batch = int(np.prod(lead)) if lead else 1
+        batch = math.prod(lead)
         out = torch.empty(lead + (ft.output_grid.size,), dtype=torch.complex128, device=t.device)
         if batch > 0:
             alpha = complex(ft._w_in_scalar) * inst.norm_factor
