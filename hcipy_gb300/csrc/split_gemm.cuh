@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                     }
                     if (g.rowmax) {
                         if (EMB && TNC > 0 && TNC % 32 == 0) {  // a warp holds columns of one row
-                            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mag));
+                            const unsigned m = __reduce_max_sync(0xffffffffu, mag > 0.0f ? __float_as_uint(mag) : 0u);  // no NaN
                             if (lane == 0 && m > 0) atomicMax(&s_rowmax[ml], m);
                         } else if (EMB) {
                             if (mag > 0.0f) atomicMax(&s_rowmax[ml], __float_as_uint(mag));
