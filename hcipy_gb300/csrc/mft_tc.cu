@@ -11,6 +11,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <atomic>
@@ -84,8 +85,8 @@ __global__ void slice_rows_kernel(FieldIO src, long long ld, int K, int Kp, cons
     }
     __syncthreads();
     const float inv = 1.0f / s_scale;
-    const long long r_cr = EMB ? (long long)m : (long long)(m / 64) * 128 + (m % 64);
-    const long long r_ci = r_cr + 64;
+    const long long r_cr = EMB ? (long long)m : (long long)(m / 16) * 32 + (m % 16);
+    const long long r_ci = r_cr + 16;
     // Four consecutive K-elements per thread: 8-byte stores into each plane (Kp and kpitch are multiples of 32).
     for (int k0 = 4 * threadIdx.x; k0 < Kp; k0 += 4 * blockDim.x) {
         __half rs[3][4], is[3][4];
@@ -469,7 +470,8 @@ struct SliceMat {
     size_t plane_bytes() const { return 3 * (size_t)rows * kpitch * sizeof(__half); }
 };
 
-int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows) {
+// bk: K-elements per box, 64 (128-byte swizzle) or 32 (64-byte swizzle)
+int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows, int bk = BK, int box_slices = NSLICE) {
     auto enc = get_encode();
     if (!enc) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -477,11 +479,12 @@ int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows) {
     }
     cuuint64_t dims[3] = {(cuuint64_t)s.kpitch, (cuuint64_t)s.rows, 3};
     cuuint64_t strides[2] = {(cuuint64_t)s.kpitch * 2, (cuuint64_t)s.rows * s.kpitch * 2};
-    cuuint32_t box[3] = {BK, (cuuint32_t)box_rows, 3};
+    cuuint32_t box[3] = {(cuuint32_t)bk, (cuuint32_t)box_rows, (cuuint32_t)box_slices};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, s.planes, dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled failed (%d) for %lld rows x %d", (int)r, s.rows, s.kpitch);
         return HX_ERR_CUDA;
@@ -734,10 +737,17 @@ int launch_choice(GemmArgs& g, const SliceMat& A, const SliceMat& B, const TileC
         set_error("split GEMM grid too large");
         return HX_ERR_UNSUPPORTED;
     }
-    HX_TRY(encode_map(&g.tmap_a, A, BM));
-    HX_TRY(encode_map(&g.tmap_b, B, c.bn));
-    g.ktiles = A.kpitch / BK;
     g.ksplit = c.ksplit;
+    // More tiles than SMs: the persistent kernel, which finishes a tile beside the next one's main loop (gradient step over
+    // 64 fields of 512^2 points 5955 -> 4883 us).  With no more tiles than SMs it has nothing to overlap (a Lyot pass over
+    // 2048^2 points 483 against 485 us) and its idle CTAs stand in the way of concurrent GEMMs (21 wavelengths on
+    // parallel graph branches 549 against 524 us).
+    const bool stream = c.bn == 128 && c.tiles > sm_count() && c.tiles <= INT_MAX && stream_fits(g);
+    const int share = stream && clusters_allowed() ? stream_share(c.n_tiles, (int)m_tiles) : 0;
+    const int bk = stream ? STREAM_BK : BK;
+    HX_TRY(share == 1 ? encode_map(&g.tmap_a, A, BM / 2, bk, 1) : encode_map(&g.tmap_a, A, BM, bk));
+    HX_TRY(share == 2 ? encode_map(&g.tmap_b, B, c.bn / 2, bk, 1) : encode_map(&g.tmap_b, B, c.bn, bk));
+    g.ktiles = A.kpitch / bk;
     g.n_tiles = c.n_tiles;
     g.partial = partial;
     g.counters = counters;
@@ -754,6 +764,7 @@ int launch_choice(GemmArgs& g, const SliceMat& A, const SliceMat& B, const TileC
     TraceScope trace(HX_TRACE_SPLIT_GEMM, cmacs, st, traced);
     if (c.bn == 64) return launch_bn64(g, grid, out, src, st);
     if (c.bn == 112) return launch_bn112(g, grid, out, src, st);
+    if (stream) return launch_stream(g, (int)m_tiles, (int)c.tiles, sm_count(), share, st);
     return launch_bn128(g, grid, out, src, st);
 }
 

@@ -131,11 +131,6 @@ template <> __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float* v
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-
 // (hi 2^24 + lo) 2^e rounded to float64 (|hi| < 2^53, |lo| < 2^48), with integer operations (the float64 pipe issues
 // about 1.6 operations per clock and SM) and without branches, so that the conversions of several columns overlap:
 // the sum's magnitude is normalised to a leading one at bit 63, rounded to 53 bits and given its exponent.  An exponent
@@ -545,7 +540,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_drained(a));
+                if (lane == 0) ptx::mbar_arrive(bar_drained(a));
             };
             level(std::integral_constant<int, 0>());
             if constexpr (S::LV > 1) {

@@ -27,8 +27,8 @@
 // (hi and lo of Re and Im); slicing reads them with FP32 operations only.
 //
 // Where the embedding lives.  When A is a plan constant (a phase matrix) the
-// embedding above is used (EMB = 0): A' holds 64-row blocks of Cr rows then Ci
-// rows and B' is the field, [Br; Bi] per column.  When A is the per-call field
+// embedding above is used (EMB = 0): A' holds 16-row blocks of Cr rows then Ci
+// rows (a warp of the epilogue then has both parts of its rows) and B' is the field, [Br; Bi] per column.  When A is the per-call field
 // (EMB = 1) the embedding moves to the constant B instead, so that the field is
 // sliced once as [Ar | Ai] (M x 2K) and never duplicated:
 //     B' = [[Br, Bi], [-Bi, Br]] (2K x 2N),  C = [Cr | Ci],
@@ -37,13 +37,13 @@
 // 128 complex rows x BN/2 complex columns, and TMEM lane = complex row.
 //
 // Kernel.  One CTA computes 64 complex rows x BN columns of C (BN = 64 or 128):
-// a 128-row tile of A' (the 64 Cr rows then their 64 Ci rows) times a BN-row
+// a 128-row tile of A' (64 Cr rows and their Ci rows) times a BN-row
 // tile of B' (EMB = 0; with EMB = 1, 128 complex rows x BN/2 complex columns).
 // warp 0 issues TMA loads (one 3-D box per operand per stage:
 // three slice planes of 64 K-elements, 128-byte swizzle), warp 1 issues
 // tcgen05.mma (8 slice products x 4 K16 steps per stage, several per MMA) into four TMEM
 // accumulators of 128 lanes x BN columns, warps 2-17 read TMEM, combine and
-// finish the result.  Three stages of 72 KiB (BN = 64) or two of 96 KiB
+// finish the result (with more tiles than SMs, the persistent form in split_gemm_stream.cu).  Three stages of 72 KiB (BN = 64) or two of 96 KiB
 // (BN = 128).  GEMMs with too few tiles to fill the GPU split K across CTAs:
 // each CTA combines its levels into a float-float partial (level 0 exactly),
 // and the partials are added in split order with float-float additions (error
@@ -190,42 +190,44 @@ __device__ __forceinline__ ff double_to_ff(double x) {
     return {hi, lo};
 }
 
-// Exact float -> float64 by bit placement (subnormal floats are normalised).
-__device__ __forceinline__ unsigned long long float_bits_to_double_bits(unsigned int fb) {
-    const unsigned long long sign = (unsigned long long)(fb & 0x80000000u) << 32;
-    const unsigned int e = (fb >> 23) & 0xff;
-    unsigned int m = fb & 0x7fffffu;
-    if (e == 0xff) return sign | 0x7ff0000000000000ull | ((unsigned long long)m << 29);
-    if (e == 0) {
-        if (m == 0) return sign;
-        const int sh = __clz(m) - 8;  // bring the leading one to bit 23
-        m = (m << sh) & 0x7fffffu;
-        return sign | ((unsigned long long)(1 - sh + 896) << 52) | ((unsigned long long)m << 29);
-    }
-    return sign | ((unsigned long long)(e + 896) << 52) | ((unsigned long long)m << 29);
-}
-
 // hi + lo as float64, rounded to nearest even.  The float64 pipe takes about 1.6 operations a clock and SM, so the sum is
 // made with integers: hi's bits placed as a float64 leave 29 zeros below, to which lo is added as a whole number of ulps
 // (lo scaled by a power of two and rounded to an int; |lo| <= ulp(hi) / 2 is 2^28 of them at most, which reaches neither
-// the exponent from below nor, with a fraction of hi that is not zero, from above).  hi below 2^-75 or beyond the floats,
-// a power of two less a lo, and pairs that are not normalised take the float64 addition; both ways give the same bits.
+// the exponent from below nor, with a fraction of hi that is not zero, from above).  hi below 2^-126 or above
+// 2^114, a power of two less a lo, and pairs that are not normalised take the float64 addition (`rare`); both ways give
+// the same bits.
+__device__ __forceinline__ double ff_to_double_fast(ff v, bool& rare) {
+    const unsigned int h = __float_as_uint(v.hi), l = __float_as_uint(v.lo);
+    const unsigned int e = (h >> 23) & 0xff;
+    const bool zero = ((h | l) << 1) == 0;
+    const float ulps = v.lo * 0x1p64f * __uint_as_float((242 - e) << 23);
+    const bool fits = e - 1 < 241 && fabsf(ulps) <= 0x1p28f && ((h & 0x7fffffu) != 0 || ((h ^ l) & 0x80000000u) == 0);
+    rare |= !fits && !zero;
+    int k = __float2int_rn(ulps);
+    if (h & 0x80000000u) k = -k;
+    const unsigned int up = (h & 0x80000000u) | (((h & 0x7fffffffu) >> 3) + (896u << 20));
+    const long long bits = (long long)(((unsigned long long)up << 32) | (h << 29)) + k;
+    return __longlong_as_double(zero ? (long long)((unsigned long long)(h & l) << 32) : bits);
+}
+
+// Both floats converted and added on the float64 pipe (volatile: not to be computed ahead of the branch that needs it).
+__device__ __forceinline__ double ff_to_double_rare(ff v) {
+    double d;
+    asm volatile(
+        "{\n\t.reg .f64 a, b;\n\tcvt.f64.f32 a, %1;\n\tcvt.f64.f32 b, %2;\n\tadd.rn.f64 %0, a, b;\n\t}"
+        : "=d"(d)
+        : "f"(v.hi), "f"(v.lo));
+    return d;
+}
+
+// One value at a time, with branches.
 __device__ __forceinline__ double ff_to_double(ff v) {
     const unsigned int h = __float_as_uint(v.hi), l = __float_as_uint(v.lo);
     if (((h | l) << 1) == 0) return __hiloint2double((int)(h & l), 0);
-    const unsigned int e = (h >> 23) & 0xff;
-    if (e >= 52 && e < 255 && ((h & 0x7fffffu) != 0 || ((h ^ l) & 0x80000000u) == 0)) {
-        const float ulps = v.lo * __uint_as_float((306 - e) << 23);
-        if (fabsf(ulps) <= 0x1p28f) {
-            int k = __float2int_rn(ulps);
-            if (h & 0x80000000u) k = -k;
-            const unsigned int up = (h & 0x80000000u) | (((h & 0x7fffffffu) >> 3) + (896u << 20));
-            const long long bits = (long long)(((unsigned long long)up << 32) | (h << 29)) + k;
-            return __longlong_as_double(bits);
-        }
-    }
-    return __dadd_rn(__longlong_as_double((long long)float_bits_to_double_bits(h)),
-                     __longlong_as_double((long long)float_bits_to_double_bits(l)));
+    bool rare = false;
+    const double d = ff_to_double_fast(v, rare);
+    if (rare) return ff_to_double_rare(v);
+    return d;
 }
 
 template <int FMT> __device__ __forceinline__ cff load_fmt(const FieldIO& f, long long i) {
@@ -345,6 +347,48 @@ __device__ __forceinline__ ff combine_levels(float v0, float v1, float v2, float
     return two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(v2 * 0x1p-34f, v3 * 0x1p-45f)));
 }
 
+// Issues the MMAs of one stage (shared-memory address `stage`; `first`: the tile's first, which starts the levels).  Called
+// by a whole warp, `leader` being its elected lane.
+// The kept products are a0 (b0 b1 b2), a1 (b0 b1 b2), a2 (b0 b1), the levels being the sums of the indices.  The
+// slices of B follow one another in shared memory as the levels do in TMEM, so one MMA multiplies a slice of
+// A by several of B: as many as 256 columns hold.  What bounds the loop is shared memory, and each MMA reads its
+// A again (4 KB): with 128 columns 5 MMAs and 52 KB per 16 K' instead of 8 and 64 KB, with 64 columns 3 and
+// 28 KB instead of 8 and 48 KB (512 x 512 outputs over 2048 points with 64 columns: 48 -> 39 us; a Lyot pass
+// over 2048^2 points 549 -> 527 us, the same bits; a stage with 128 columns now takes 2220 clocks, its MMAs
+// 2048).  The order of the products within a level is that of the single ones.
+template <int BN, int ROW = 2 * BK>
+__device__ __forceinline__ void slice_products(uint32_t tmem, uint32_t stage, bool first, bool leader) {
+    // descriptors of a K-major operand whose rows are ROW bytes wide and swizzled over that width: 8-row groups
+    // 8 ROW bytes apart, version 1, swizzle mode 2 (128 bytes) or 4 (64)
+    static_assert(ROW == 128 || ROW == 64, "128- or 64-byte swizzle");
+    constexpr uint32_t desc_hi = (8u * ROW >> 4) | (1u << 14) | ((ROW == 128 ? 2u : 4u) << 29);
+    constexpr int MAXS = 256 / BN < NSLICE ? 256 / BN : NSLICE;  // slices of B per MMA
+    const uint32_t a0 = ((stage & 0x3FFFF) >> 4) | (1u << 16);
+    const uint32_t b0 = a0 + (NSLICE * BM * ROW >> 4);
+    auto mma = [&](auto count, int pa, int pb, int kk, bool start) {
+        constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN * decltype(count)::value);
+        if (leader)
+            ptx::umma_f16_lo(tmem + (pa + pb) * BN, a0 + ((pa * BM * ROW + kk * 32) >> 4),
+                             b0 + ((pb * BN * ROW + kk * 32) >> 4), desc_hi, idesc, start);
+    };
+    using one = std::integral_constant<int, 1>;
+    using two = std::integral_constant<int, 2>;
+    using most = std::integral_constant<int, MAXS>;
+#pragma unroll
+    for (int kk = 0; kk < ROW / 32; ++kk) {
+        const bool start = first && kk == 0;  // the first product of a level starts it
+        mma(most{}, 0, 0, kk, start);
+        if (MAXS < 3) mma(one{}, 0, 2, kk, start);
+        if (MAXS < 3 || start) {  // a1 b2 starts level 3
+            mma(two{}, 1, 0, kk, false);
+            mma(one{}, 1, 2, kk, start);
+        } else {
+            mma(most{}, 1, 0, kk, false);
+        }
+        mma(two{}, 2, 0, kk, false);
+    }
+}
+
 // OUT: format of the result; SRC: format of the Babinet source (FMT_NONE for other epilogues); EMB: where the
 // complex embedding lives (0: on A, 1: on B).
 template <int BN, int OUT, int SRC, int EMB>
@@ -441,17 +485,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         // The whole warp runs this branch with only the instructions themselves under the elected lane: issued from a
         // one-lane branch, with 64-bit descriptors built for each, an MMA took 79 clocks of the issuing thread where
         // the 128-column product itself takes 64.
-        // descriptors of a K-major operand with 128-byte swizzle: 8-row groups 1024 B apart, version 1, swizzle mode 2
-        constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
         const bool leader = ptx::elect_one();
-        // The kept products are a0 (b0 b1 b2), a1 (b0 b1 b2), a2 (b0 b1), the levels being the sums of the indices.  The
-        // slices of B follow one another in shared memory as the levels do in TMEM, so one MMA multiplies a slice of
-        // A by several of B: as many as 256 columns hold.  What bounds the loop is shared memory, and each MMA reads its
-        // A again (4 KB): with 128 columns 5 MMAs and 52 KB per 16 K' instead of 8 and 64 KB, with 64 columns 3 and
-        // 28 KB instead of 8 and 48 KB (512 x 512 outputs over 2048 points with 64 columns: 48 -> 39 us; a Lyot pass
-        // over 2048^2 points 549 -> 527 us, the same bits; a stage with 128 columns now takes 2220 clocks, its MMAs
-        // 2048).  The order of the products within a level is that of the single ones.
-        constexpr int MAXS = 256 / BN < NSLICE ? 256 / BN : NSLICE;  // slices of B per MMA
         bool ok = true;
         for (int i = 0; i < nkt; ++i) {
             const int s = i % STAGES;
@@ -459,30 +493,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
             ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, WAIT_LIMIT));
             if (!ok) break;
             ptx::tc_fence_after();
-            const uint32_t a0 = (((smem_base + s * T::STAGE_BYTES) & 0x3FFFF) >> 4) | (1u << 16);
-            const uint32_t b0 = a0 + (A_STAGE_BYTES >> 4);
-            auto mma = [&](auto count, int pa, int pb, int kk, bool start) {
-                constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, BN * decltype(count)::value);
-                if (leader)
-                    ptx::umma_f16_lo(tmem + (pa + pb) * BN, a0 + ((pa * A_PLANE_BYTES + kk * 32) >> 4),
-                                     b0 + ((pb * T::B_PLANE_BYTES + kk * 32) >> 4), desc_hi, idesc, start);
-            };
-            using one = std::integral_constant<int, 1>;
-            using two = std::integral_constant<int, 2>;
-            using most = std::integral_constant<int, MAXS>;
-#pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                const bool start = i == 0 && kk == 0;  // the first product of a level starts it
-                mma(most{}, 0, 0, kk, start);
-                if (MAXS < 3) mma(one{}, 0, 2, kk, start);
-                if (MAXS < 3 || start) {  // a1 b2 starts level 3
-                    mma(two{}, 1, 0, kk, false);
-                    mma(one{}, 1, 2, kk, start);
-                } else {
-                    mma(most{}, 1, 0, kk, false);
-                }
-                mma(two{}, 2, 0, kk, false);
-            }
+            slice_products<BN>(tmem, smem_base + s * T::STAGE_BYTES, i == 0, leader);
             if (leader) ptx::umma_commit(bar_empty(s));
         }
         // Arrives once every MMA issued above has completed (at once if none was issued); TMEM is
@@ -676,28 +687,30 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
         const bool run = finish && live && !*abort_flag;
         const int ncol0 = n_tile * TN + q * TNs;  // first complex column of the slice
         // The rows of the slice: with the whole tile (no cluster) its width is a compile-time constant.
-        auto rows_pass = [&](auto tns_c) {
+        const cff alpha = {{g.alpha[0], g.alpha[1]}, {g.alpha[2], g.alpha[3]}};
+        const bool real_alpha = g.alpha[2] == 0.0f && g.alpha[3] == 0.0f;
+        const bool imag_alpha = g.alpha[0] == 0.0f && g.alpha[1] == 0.0f;  // e.g. Fraunhofer's 1/(i f lambda)
+        const bool unit_alpha = real_alpha && g.alpha[0] == 1.0f && g.alpha[1] == 0.0f;
+        auto rows_pass = [&](auto tns_c, auto times_alpha) {
             constexpr int TNC = decltype(tns_c)::value;
             const int TNS = TNC > 0 ? TNC : TNs;
-            const cff alpha = {{g.alpha[0], g.alpha[1]}, {g.alpha[2], g.alpha[3]}};
-            const bool real_alpha = g.alpha[2] == 0.0f && g.alpha[3] == 0.0f;
-            const bool imag_alpha = g.alpha[0] == 0.0f && g.alpha[1] == 0.0f;  // e.g. Fraunhofer's 1/(i f lambda)
-            const bool unit_alpha = real_alpha && g.alpha[0] == 1.0f && g.alpha[1] == 0.0f;
             const float2* mask = (g.epi == HX_EPI_MUL || g.epi == HX_EPI_BABINET) ? g.mask : nullptr;
             // Each thread keeps one complex column of the slice; a warp covers consecutive columns of one row.
             const int nl = et % TNS;
             const int n = ncol0 + nl;
             const bool nok = n < g.N;
             const float csc = nok ? g.col_scale[z * g.col_scale_z + n] : 0.0f;
-            // staged position of the real and imaginary parts: EMB = 0, rows ml and 64 + ml of column nl;
+            // staged position of the real and imaginary parts: EMB = 0, the rows of the 16-row Cr / Ci blocks, column nl;
             // EMB = 1, row ml, columns of the 8-column Cr / Ci blocks
             const int c_re = EMB ? (nl >> 3) * 16 + (nl & 7) : nl;
             const int c_im = EMB ? c_re + 8 : nl;
-            constexpr int R_IM = EMB ? 0 : 64;
+            constexpr int R_IM = EMB ? 0 : 16;
+            auto r_re = [](int ml) { return EMB ? ml : (ml >> 4) * 32 + (ml & 15); };
             // rows per iteration: a power of two, so that whole iterations make up the tile's rows
             const int RSTEP = min(TM, 1 << (31 - __clz(EPI / TNS)));
             const int ITER = TM / RSTEP;
-            constexpr int U = 4;                  // rows per batch: loads issued before any store
+            // rows per batch: loads issued before any store (two where they are converted to float64, see below)
+            constexpr int U = OUT == FMT_C128 ? 2 : 4;
             // Threads past RSTEP * TNs (BN = 112) have no column; they skip the loop so that no row beyond the tile's
             // TM is touched.
             const bool has_col = et < RSTEP * TNS;
@@ -726,12 +739,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                     float mag = 0.0f;
                     if (nok && ml < mlim) {
                         const float sc = s_rscale[ml] * csc;  // product of powers of two: exact
-                        cff v = {ff{fin_hi[ml * fpitch + c_re] * sc, fin_lo[ml * fpitch + c_re] * sc},
-                                 ff{fin_hi[(R_IM + ml) * fpitch + c_im] * sc, fin_lo[(R_IM + ml) * fpitch + c_im] * sc}};
-                        if (!unit_alpha)
-                            v = real_alpha   ? cff{ff_mul(v.re, alpha.re), ff_mul(v.im, alpha.re)}
-                                : imag_alpha ? cff{ff_neg(ff_mul(v.im, alpha.im)), ff_mul(v.re, alpha.im)}
-                                             : cff_mul(v, alpha);
+                        const int o_re = r_re(ml) * fpitch + c_re, o_im = (R_IM + r_re(ml)) * fpitch + c_im;
+                        cff v = {ff{fin_hi[o_re] * sc, fin_lo[o_re] * sc}, ff{fin_hi[o_im] * sc, fin_lo[o_im] * sc}};
+                        v = times_alpha(v);
                         if constexpr (SRC != FMT_NONE) v = {ff_add(e[u].re, ff_neg(v.re)), ff_add(e[u].im, ff_neg(v.im))};
                         if (mask) v = mk[u].y == 0.0f ? cff{ff_mulf(v.re, mk[u].x), ff_mulf(v.im, mk[u].x)}
                                                       : cff_mul_c64(v, mk[u]);
@@ -765,8 +775,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) split_gemm_kernel(const __grid
                 atomicMax(&g.colmax[z * g.colmax_z + cfield * g.colmax_field_stride + n], __float_as_uint(cmax));
         };
         if (run) {
-            if (S == 1) rows_pass(std::integral_constant<int, TN>{});
-            else rows_pass(std::integral_constant<int, 0>{});
+            // One loop for each kind of factor, so that a launch runs through the code of its own only: the kinds side by
+            // side, four rows at a time, overflowed the instruction cache (Lyot pass over 2048^2 points 512 -> 485 us).
+            auto rows = [&](auto tns_c) {
+                if (unit_alpha) rows_pass(tns_c, [](cff x) { return x; });
+                else if (real_alpha)
+                    rows_pass(tns_c, [&](cff x) { return cff{ff_mul(x.re, alpha.re), ff_mul(x.im, alpha.re)}; });
+                else if (imag_alpha)
+                    rows_pass(tns_c, [&](cff x) { return cff{ff_neg(ff_mul(x.im, alpha.im)), ff_mul(x.re, alpha.im)}; });
+                else rows_pass(tns_c, [&](cff x) { return cff_mul(x, alpha); });
+            };
+            if (S == 1) rows(std::integral_constant<int, TN>{});
+            else rows(std::integral_constant<int, 0>{});
         }
         ptx::named_barrier(1, EPI);
         if (run && g.rowmax && et < TM && et < g.M - m_tile * TM) {
@@ -882,6 +902,14 @@ template <int BN> int cluster_ok(int ksplit) {
 int launch_bn64(const GemmArgs& g, dim3 grid, int out, int src, cudaStream_t st);
 int launch_bn112(const GemmArgs& g, dim3 grid, int out, int src, cudaStream_t st);
 int launch_bn128(const GemmArgs& g, dim3 grid, int out, int src, cudaStream_t st);
+
+// Persistent form of the 128-column tiles (split_gemm_stream.cu): whether it takes this GEMM, and its launch.
+constexpr int STREAM_BK = 32;  // K' elements per stage
+bool stream_fits(const GemmArgs& g);
+// Which operand pairs of its CTAs share: 0 none, 1 A (neighbouring column tiles), 2 B (neighbouring row tiles).  The shared
+// operand's boxes are 64 rows of one slice.
+int stream_share(int n_tiles, int m_tiles);
+int launch_stream(const GemmArgs& g, int m_tiles, int tiles, int ctas, int share, cudaStream_t st);
 
 }  // namespace sg
 }  // namespace hx
