@@ -69,6 +69,18 @@ int launch_shape(int M, const std::vector<int>& radices, int nlines, int batch, 
         lpc = (int)std::max<long long>(std::min<long long>(lpc, std::max<long long>(lines_needed, min_lines)), 1);
     }
     lpc = std::min(lpc, nlines);
+    if (sizeof(T) == 8) {
+        // float64 lines are bound by the float64 pipe, so a pass takes as long as the SM with the most lines: fewer lines
+        // per CTA where that evens them out by a tenth or more, though neighbouring lines are then loaded by several
+        // CTAs.  360^2 points backward 60 -> 50 us, 256^2 in 512^2 95 -> 54, 512^2 99 -> 70, 1024^2 277 -> 228 us.  With many
+        // lines per SM the loads are even already and the wider segments count (16 fields of 100^2: 50 against 52 us).
+        const long long sms = num_sms();
+        auto most = [&](int l) { return (((nlines + l - 1) / l * (long long)batch + sms - 1) / sms) * l; };
+        int best = lpc;
+        for (int l = lpc - 1; l >= 1; --l)
+            if (most(l) <= most(best)) best = l;
+        if (10 * most(best) <= 9 * most(lpc)) lpc = best;
+    }
     const int ppt = mixed ? Ppt<T, true>::value : Ppt<T, false>::value;
     auto threads_for = [&](int lines) {
         int need = 32;
