@@ -465,13 +465,15 @@ template <typename T> int fields_per_pass(const Dims& d, int batch) {
     return (int)std::max<long long>(1, std::min<long long>({batch, rows, (long long)(((size_t)4 << 30) / one)}));
 }
 
-// Where the tensor-core form is the faster one: below these complex multiply-adds its four launches (about 35 us on
-// the device) cost more than the products on the CUDA cores.  complex64: 512^2 -> 256^2 (1.0e8) 59 us against 81, at
-// 3e7 both take 50; complex128: two fields 100 x 90 <- 70 x 40 (1.8e6) 95 us against 128, 512^2 -> 256^2 78 against 1072.
+// Where the tensor-core form is the faster one, transforms that the one-launch form takes aside: its four launches take 33
+// to 45 us however small.  On the CUDA cores a pair of GEMMs takes 0.075 us for each term of its two sums (one after
+// the other: 384^2 -> 192^2 60 us, 700^2 -> 100^2 103 us, 1001 x 501 -> 33^2 109 us in complex64), or what its products
+// take where they are many and the sums short (700^2 <- 100^2, 5.6e7 products, 31 us).  complex128 there waits for the
+// float64 pipe: 50^2 -> 50^2 (2.5e5 products) 123 us against 42, 16 fields of 64^2 -> 32^2 141 against 45.
 template <typename T> bool takes(const Dims& d, int batch) {
     if (std::min(std::min(d.K1, d.K2), std::min(d.R, d.C)) < 16) return false;
     const double cmacs = (double)batch * ((double)d.K1 * d.K2 * d.C + (double)d.R * d.K1 * d.C);
-    return cmacs >= (sizeof(T) == 4 ? 6e7 : 1.5e6);
+    return sizeof(T) == 4 ? cmacs >= 6e7 || d.K1 + d.K2 >= 600 : cmacs >= 1e5;
 }
 
 template <typename T> int make_const(PlaneMat& m, int N, const double* a, const double* b, double sign,
