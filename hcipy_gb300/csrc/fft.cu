@@ -1,6 +1,7 @@
 // FFT-family plans: the zero-padded FastFourierTransform, the Fourier filter
 // (FourierFilter / angular-spectrum and Fresnel propagation), the chirp-Z transform, and the
-// angular-spectrum and Fresnel transfer functions.  All transforms run fft_line_kernel.
+// angular-spectrum and Fresnel transfer functions.  complex64 lines of 256 to 4096 points (powers of two) run
+// fft_pow2_kernel, all others fft_line_kernel.
 //
 // Reference behaviour restated here:
 //   FastFourierTransform  hcipy/fourier/fast_fourier_transform.py:223-406

@@ -21,7 +21,8 @@
 //   out[l, kk] = buf[src] * chirp_out[src] * post[l, kk] * scale
 // This one kernel serves the zero-padded FFT with fftshifts and crop, the
 // chirp-Z transform (Bluestein), Bluestein for lengths that are not
-// 2,3,5,7-smooth, and the column pass of the Fourier filter.
+// 2,3,5,7-smooth, and the column pass of the Fourier filter, for every line that
+// fft_pow2.cuh does not take.
 #pragma once
 
 #include "hx_common.cuh"

@@ -16,8 +16,12 @@
 //
 // Sums.  The tensor cores truncate an FP32 sum that no longer fits 24 bits (a sum of 4096 positive
 // products comes out 2.5e-5 low, of 64 products 1.5e-7 low: measured against float64), so no accumulator runs long:
-//   complex64 : 32 terms of K' (6.5e-8 low), then the accumulator is added to FP32 registers in round-to-nearest, in
-//               blocks of 16 partial sums;
+//   complex64 : 32 terms of K', then the accumulator is added to FP32 registers in round-to-nearest, in blocks of 16
+//               partial sums.  Such a sum is truncated after its first 16 terms and at the end, by half an ulp on
+//               average: 2^-24 / (2 ln 2) = 4.3e-8 of a value with mantissas spread over their logarithm, and half of
+//               that for the first truncation, 6.4e-8 together (6.5e-8 measured), whatever the signs of the terms.
+//               A factor so close to 1 on every GEMM adds up along a chain of transforms, so it is taken back on
+//               average (Sums<float>::add);
 //   complex128: 128 terms: every level is then an integer below 7 * 128 * 2^14 < 2^24, hence exact, and is added to
 //               64-bit integers (levels 0-3 in one, 4-6 in another), exact over any K the plans take.
 // The error of a complex128 transform is that of its operands (2^-56 of a row maximum) and of the dropped products
@@ -196,9 +200,12 @@ template <> struct Sums<float> {
 #pragma unroll
         for (int j = 0; j < COLS; ++j) tot[j] = blk[j] = 0.0f;
     }
+    // Every second partial sum times 1 + 2^-23, in the one rounding of the addition: 6.0e-8 of the 6.4e-8 that the
+    // truncated sums lose on average (see above).
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
+        const float w = (n & 1) ? 1.0f : 1.0f + 0x1p-23f;
 #pragma unroll
-        for (int j = 0; j < Layout<float>::LD; ++j) blk[j0 + j] += v[j];
+        for (int j = 0; j < Layout<float>::LD; ++j) blk[j0 + j] = fmaf(v[j], w, blk[j0 + j]);
     }
     __device__ __forceinline__ void end_partial(bool last) {
         if ((++n & 15) != 0 && !last) return;

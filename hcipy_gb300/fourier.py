@@ -197,7 +197,8 @@ class MatrixFourierTransform(FourierTransform):
     """Matrix Fourier transform (hcipy/fourier/matrix_fourier_transform.py:8-310) as two device GEMMs.
 
     ``precision`` selects the GEMM arithmetic: ``'fp32'`` (default) is the plain
-    drop-in (complex64 fields on FP32 CUDA cores, complex128 fields in FP64);
+    drop-in (complex64 and complex128 accuracy; on the tensor cores where the transform is large enough for them, else
+    in FP32 and FP64 arithmetic);
     ``'split'`` runs on tcgen05 tensor cores with fixed-point fp16 slices and
     exact sums (~29-bit operands), takes complex64 or complex128 fields and
     returns complex128, since its results hold more than a complex64 can.  ``precompute_matrices`` and
