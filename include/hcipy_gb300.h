@@ -55,7 +55,8 @@ extern "C" {
 #define HX_ADJOINT 2  /* the conjugate transpose of forward (input weights); used by gradients */
 
 /* Arithmetic of the MFT GEMMs. */
-#define HX_PREC_FP32 0  /* FP32 CUDA-core complex GEMM (HX_C64) or FP64 (HX_C128) */
+#define HX_PREC_FP32 0  /* the field's own precision, FP32 (HX_C64) or FP64 (HX_C128): tensor-core GEMMs of fp16
+                           planes, CUDA-core GEMMs for transforms too small for them */
 #define HX_PREC_SPLIT 1 /* split-operand tensor-core GEMM on tcgen05 (grids up to 8192 points per axis) */
 
 /* Tile policy of a plan's GEMMs (no counterpart in the reference). */
@@ -75,7 +76,7 @@ HX_API long long hx_launch_count(void);
  * hx_trace_read waits for the recorded events of one kernel family and returns launches, summed device time
  * and summed work since the last reset. */
 #define HX_TRACE_SPLIT_GEMM 0 /* split-operand tcgen05 GEMM of the MFT */
-#define HX_TRACE_SIMT_GEMM 1  /* CUDA-core complex GEMM of the MFT (FP32 or FP64) */
+#define HX_TRACE_SIMT_GEMM 1  /* complex GEMM of the MFT in FP32 or FP64 (CUDA cores or fp16 planes) */
 #define HX_TRACE_FFT 2        /* line-FFT passes (FFT, filter, chirp-Z) */
 #define HX_TRACE_ATMOSPHERE 3 /* screen extrusion and sub-pixel shift (work = bytes) */
 #define HX_TRACE_DM 4         /* influence-function products and phase screens (work = bytes) */
@@ -104,7 +105,9 @@ HX_API int hx_mft_plan_create(int nx, int ny, int nu, int nv,
                        const double* w_out_u, const double* w_out_v,
                        int dtype, int precision, void* stream, hx_mft_plan** plan);
 
-/* Bytes of caller-provided scratch that hx_mft_execute needs for `batch` fields. */
+/* Bytes of caller-provided scratch that hx_mft_execute wants for `batch` fields.  Given less, down to the intermediate
+ * field of the two GEMMs (batch x ny x nu elements), FP32 and FP64 plans run on the CUDA cores instead of the tensor
+ * cores; below that the call is refused. */
 HX_API size_t hx_mft_workspace_bytes(const hx_mft_plan* plan, int direction, int batch);
 
 /* `in` holds `batch` contiguous fields of the source plane, `out` receives
@@ -195,8 +198,8 @@ HX_API int hx_mft_plan_status(const hx_mft_plan* plan, int reset);
  * transforms run concurrently with others (several streams, or parallel branches of a CUDA graph): small
  * transforms then take the tile with the least SM time instead of splitting K to fill the GPU alone (a split
  * tensor-core GEMM still splits a contraction longer than 4096 real terms, to keep its sums exact), and the
- * autotuner's measurements are ranked by duration x occupied SMs; FP32/FP64 plans keep their widest CUDA-core
- * tile instead of narrowing it to occupy the GPU. */
+ * autotuner's measurements are ranked by duration x occupied SMs; FP32/FP64 plans neither split K nor narrow
+ * their CUDA-core tile to occupy the GPU. */
 HX_API int hx_mft_plan_set_schedule(hx_mft_plan* plan, int schedule);
 
 /* Tile autotuner of the split tensor-core GEMMs (process-wide; no counterpart in the reference).  When on,
