@@ -471,7 +471,7 @@ struct SliceMat {
 };
 
 // bk: K-elements per box, 64 (128-byte swizzle) or 32 (64-byte swizzle)
-int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows, int bk = BK, int box_slices = NSLICE) {
+int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows, int bk = BK) {
     auto enc = get_encode();
     if (!enc) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -479,7 +479,7 @@ int encode_map(CUtensorMap* map, const SliceMat& s, int box_rows, int bk = BK, i
     }
     cuuint64_t dims[3] = {(cuuint64_t)s.kpitch, (cuuint64_t)s.rows, 3};
     cuuint64_t strides[2] = {(cuuint64_t)s.kpitch * 2, (cuuint64_t)s.rows * s.kpitch * 2};
-    cuuint32_t box[3] = {(cuuint32_t)bk, (cuuint32_t)box_rows, (cuuint32_t)box_slices};
+    cuuint32_t box[3] = {(cuuint32_t)bk, (cuuint32_t)box_rows, NSLICE};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, s.planes, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -739,14 +739,13 @@ int launch_choice(GemmArgs& g, const SliceMat& A, const SliceMat& B, const TileC
     }
     g.ksplit = c.ksplit;
     // More tiles than SMs: the persistent kernel, which finishes a tile beside the next one's main loop (gradient step over
-    // 64 fields of 512^2 points 5955 -> 4883 us).  With no more tiles than SMs it has nothing to overlap (a Lyot pass over
+    // 64 fields of 512^2 points 5955 -> 4947 us).  With no more tiles than SMs it has nothing to overlap (a Lyot pass over
     // 2048^2 points 483 against 485 us) and its idle CTAs stand in the way of concurrent GEMMs (21 wavelengths on
     // parallel graph branches 549 against 524 us).
     const bool stream = c.bn == 128 && c.tiles > sm_count() && c.tiles <= INT_MAX && stream_fits(g);
-    const int share = stream && clusters_allowed() ? stream_share(c.n_tiles, (int)m_tiles) : 0;
     const int bk = stream ? STREAM_BK : BK;
-    HX_TRY(share == 1 ? encode_map(&g.tmap_a, A, BM / 2, bk, 1) : encode_map(&g.tmap_a, A, BM, bk));
-    HX_TRY(share == 2 ? encode_map(&g.tmap_b, B, c.bn / 2, bk, 1) : encode_map(&g.tmap_b, B, c.bn, bk));
+    HX_TRY(encode_map(&g.tmap_a, A, BM, bk));
+    HX_TRY(encode_map(&g.tmap_b, B, c.bn, bk));
     g.ktiles = A.kpitch / bk;
     g.n_tiles = c.n_tiles;
     g.partial = partial;
@@ -764,7 +763,7 @@ int launch_choice(GemmArgs& g, const SliceMat& A, const SliceMat& B, const TileC
     TraceScope trace(HX_TRACE_SPLIT_GEMM, cmacs, st, traced);
     if (c.bn == 64) return launch_bn64(g, grid, out, src, st);
     if (c.bn == 112) return launch_bn112(g, grid, out, src, st);
-    if (stream) return launch_stream(g, (int)m_tiles, (int)c.tiles, sm_count(), share, st);
+    if (stream) return launch_stream(g, (int)m_tiles, (int)c.tiles, sm_count(), st);
     return launch_bn128(g, grid, out, src, st);
 }
 

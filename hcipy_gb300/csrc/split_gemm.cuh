@@ -906,10 +906,7 @@ int launch_bn128(const GemmArgs& g, dim3 grid, int out, int src, cudaStream_t st
 // Persistent form of the 128-column tiles (split_gemm_stream.cu): whether it takes this GEMM, and its launch.
 constexpr int STREAM_BK = 32;  // K' elements per stage
 bool stream_fits(const GemmArgs& g);
-// Which operand pairs of its CTAs share: 0 none, 1 A (neighbouring column tiles), 2 B (neighbouring row tiles).  The shared
-// operand's boxes are 64 rows of one slice.
-int stream_share(int n_tiles, int m_tiles);
-int launch_stream(const GemmArgs& g, int m_tiles, int tiles, int ctas, int share, cudaStream_t st);
+int launch_stream(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st);
 
 }  // namespace sg
 }  // namespace hx

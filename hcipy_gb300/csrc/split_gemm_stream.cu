@@ -13,7 +13,7 @@
 //
 // What it measured: GEMMs of 64 stacked fields, 512^2 points to 512^2, complex64-to-float-float 395 -> 296 us, and with
 // complex128 results from 256 points 319 -> 194 us; a gradient step through a Lyot coronagraph over 64 fields of 512^2
-// points 5955 -> 4883 us.  A tile of 16 K steps of 64 takes 36 to 39 thousand clocks, 33 of them MMAs: what is left is the
+// points 5955 -> 4947 us.  A tile of 16 K steps of 64 takes 36 to 39 thousand clocks, 33 of them MMAs: what is left is the
 // 2 thousand in which the levels are read (TMEM holds one tile's) and loads that the stores delay.
 // On the way there: the loads alone take 23 thousand clocks a tile, so neither they nor L2 bound the loop; the epilogue
 // did, through instructions (see `scale` and store_rows), and through stores that touched 32 lines each.
@@ -143,13 +143,10 @@ __device__ __forceinline__ float column_max(float (&mag)[16], int lane) {
     return mag[0];
 }
 
-// SHARE: 1, the two CTAs of a cluster take neighbouring column tiles and share A; 2, neighbouring row tiles and share B;
-// 0, no cluster.  Each CTA loads half of the shared operand into both, which takes a quarter off the reads from L2 (360 to
-// 374 us where A is a constant; where it is the field, within 2%).
-template <int OUT, int EMB, int SHARE>
+// Every CTA loads both operands of its tiles itself, mostly from L2.
+template <int OUT, int EMB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     split_stream_kernel(const __grid_constant__ GemmArgs g, int m_tiles, int tiles) {
-    constexpr int CTAS = SHARE ? 2 : 1;
     constexpr int TM = EMB ? 128 : 64;
     constexpr int TN = EMB ? SBN / 2 : SBN;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -170,7 +167,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             ptx::mbar_init(bar_full(s), 1);
-            ptx::mbar_init(bar_empty(s), CTAS);  // a stage is refilled when every CTA it goes to has used it
+            ptx::mbar_init(bar_empty(s), 1);
         }
         ptx::mbar_init(bar_accum, 1);
         ptx::mbar_init(bar_drained, EPI_WARPS);
@@ -183,20 +180,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
-    if (SHARE) ptx::cluster_sync();  // the other CTA's copies and commits find this one's barriers
-    else __syncthreads();
+    __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t smem_base = ptx::smem_addr(smem);
     const int nkt = g.ktiles;
-    const int rank = SHARE ? (int)ptx::cluster_rank() : 0;
-    // The work items of a cluster: a tile, or two neighbouring ones of which this CTA takes the rank-th.
-    const int nw = SHARE == 1 ? g.n_tiles / 2 : g.n_tiles, mw = SHARE == 2 ? m_tiles / 2 : m_tiles;
-    const int item0 = blockIdx.x / CTAS, items = tiles / CTAS, step = gridDim.x / CTAS;
+    const int tile0 = blockIdx.x, step = gridDim.x;
     auto place = [&](int t, int& n_tile, int& m_tile, int& z) {
-        n_tile = SHARE == 1 ? t % nw * 2 + rank : t % nw;
-        m_tile = SHARE == 2 ? t / nw % mw * 2 + rank : t / nw % mw;
-        z = t / nw / mw;
+        n_tile = t % g.n_tiles;
+        m_tile = t / g.n_tiles % m_tiles;
+        z = t / g.n_tiles / m_tiles;
     };
 
     if (warp == 0) {
@@ -204,7 +197,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             int last_use[STAGES];
             for (int s = 0; s < STAGES; ++s) last_use[s] = -1;
             int it = 0;
-            for (int t = item0; t < items && !*abort_flag; t += step) {
+            for (int t = tile0; t < tiles && !*abort_flag; t += step) {
                 int n_tile, m_tile, z;
                 place(t, n_tile, m_tile, z);
                 const int a_row0 = m_tile * BM + z * g.a_rows_per_z;
@@ -219,18 +212,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                     uint8_t* sa = smem + s * STAGE;
                     uint8_t* sb = sa + STAGE_A;
                     ptx::mbar_arrive_expect_tx(bar_full(s), STAGE);
-                    // the shared operand: this CTA's half of the rows of each slice, into both
-                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int row0, bool shared) {
-                        if (!shared) {
-                            ptx::tma_load_3d(ptx::smem_addr(dst), map, i * STREAM_BK, row0, 0, bar_full(s));
-                            return;
-                        }
-                        for (int p = 0; p < NSLICE; ++p)
-                            ptx::tma_load_3d_multicast(ptx::smem_addr(dst) + (p * BM + rank * (BM / 2)) * ROW_BYTES, map,
-                                                       i * STREAM_BK, row0 + rank * (BM / 2), p, bar_full(s), 3);
-                    };
-                    load(sa, &g.tmap_a, a_row0, SHARE == 1);
-                    load(sb, &g.tmap_b, b_row0, SHARE == 2);
+                    ptx::tma_load_3d(ptx::smem_addr(sa), &g.tmap_a, i * STREAM_BK, a_row0, 0, bar_full(s));
+                    ptx::tma_load_3d(ptx::smem_addr(sb), &g.tmap_b, i * STREAM_BK, b_row0, 0, bar_full(s));
                     last_use[s] = u;
                 }
             }
@@ -238,17 +221,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             for (int s = 0; s < STAGES; ++s)
                 if (last_use[s] >= 0 && !ptx::mbar_wait_bounded(bar_full(s), last_use[s] & 1, WAIT_LIMIT))
                     raise_status(g.status, abort_flag);
-            // Nor an arrival of the other CTA's MMAs.
-            for (int s = 0; SHARE && s < STAGES; ++s)
-                if (last_use[s] >= 0 && !ptx::mbar_wait_bounded(bar_empty(s), last_use[s] & 1, WAIT_LIMIT))
-                    raise_status(g.status, abort_flag);
         }
         __syncwarp();
     } else if (warp == 1) {
         const bool leader = ptx::elect_one();
         bool ok = true;
         int it = 0, j = 0;
-        for (int t = item0; t < items && ok; t += step, ++j) {
+        for (int t = tile0; t < tiles && ok; t += step, ++j) {
             if (j > 0) ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained, (j - 1) & 1, WAIT_LIMIT));
             ptx::tc_fence_after();
             for (int i = 0; i < nkt && ok; ++i, ++it) {
@@ -257,10 +236,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                 if (!ok) break;
                 ptx::tc_fence_after();
                 slice_products<SBN, ROW_BYTES>(tmem, smem_base + s * STAGE, i == 0, leader);
-                if (leader) {
-                    if (SHARE) ptx::umma_commit_multicast(bar_empty(s), 3);
-                    else ptx::umma_commit(bar_empty(s));
-                }
+                if (leader) ptx::umma_commit(bar_empty(s));
             }
             if (!ok && leader) raise_status(g.status, abort_flag);
             if (leader) ptx::umma_commit(bar_accum);
@@ -281,7 +257,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         const float2* mask = g.epi == HX_EPI_MUL ? g.mask : nullptr;
         const bool mask_pairs = g.N % 2 == 0 && (reinterpret_cast<uintptr_t>(mask) & 15) == 0;
         int j = 0;
-        for (int t = item0; t < items; t += step, ++j) {
+        for (int t = tile0; t < tiles; t += step, ++j) {
             int n_tile, m_tile, z;
             place(t, n_tile, m_tile, z);
             // this thread's row and its 16 columns
@@ -394,18 +370,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     }
     ptx::tc_fence_before();
     __syncwarp();
-    if (SHARE) ptx::cluster_sync();  // neither CTA leaves while the other's copies or commits may reach it
-    else __syncthreads();
+    __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem, TMEM_COLS);
     }
 }
 
-template <int OUT, int EMB, int SHARE>
-int launch(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st) {
+template <int OUT, int EMB> int launch(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st) {
     static bool configured[64];
-    auto kern = split_stream_kernel<OUT, EMB, SHARE>;
+    auto kern = split_stream_kernel<OUT, EMB>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
@@ -413,33 +387,12 @@ int launch(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st)
                            "cudaFuncSetAttribute(split_stream_kernel)"));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(SHARE ? ctas & ~1 : ctas));
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = SHARE ? 1 : 0;
-    HX_TRY(cuda_status(cudaLaunchKernelEx(&cfg, kern, g, m_tiles, tiles), "split_stream_kernel"));
+    kern<<<(unsigned)ctas, NUM_THREADS, SMEM, st>>>(g, m_tiles, tiles);
     return launch_status("split_stream_kernel");
 }
 
-template <int OUT, int EMB> int launch_share(const GemmArgs& g, int m_tiles, int tiles, int ctas, int share, cudaStream_t st) {
-    switch (share) {
-        case 1: return launch<OUT, EMB, 1>(g, m_tiles, tiles, ctas, st);
-        case 2: return launch<OUT, EMB, 2>(g, m_tiles, tiles, ctas, st);
-        default: return launch<OUT, EMB, 0>(g, m_tiles, tiles, ctas, st);
-    }
-}
-
-template <int OUT> int launch_emb(const GemmArgs& g, int m_tiles, int tiles, int ctas, int share, cudaStream_t st) {
-    return g.emb ? launch_share<OUT, 1>(g, m_tiles, tiles, ctas, share, st)
-                 : launch_share<OUT, 0>(g, m_tiles, tiles, ctas, share, st);
+template <int OUT> int launch_emb(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st) {
+    return g.emb ? launch<OUT, 1>(g, m_tiles, tiles, ctas, st) : launch<OUT, 0>(g, m_tiles, tiles, ctas, st);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -457,39 +410,11 @@ bool stream_fits(const GemmArgs& g) {
     }
 }
 
-int stream_share(int n_tiles, int m_tiles) {
-    static int cache[64];  // per device: 0 unknown, 1 two CTAs fit a cluster, 2 they do not
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (cache[dev] == 0) {
-        auto kern = split_stream_kernel<FMT_FF, 0, 1>;
-        int n = 0;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2);
-        cfg.blockDim = dim3(NUM_THREADS);
-        cfg.dynamicSmemBytes = SMEM;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const bool ok =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
-        cudaGetLastError();  // a refused query leaves no error behind
-        cache[dev] = ok ? 1 : 2;
-    }
-    if (cache[dev] != 1) return 0;
-    return n_tiles % 2 == 0 ? 1 : m_tiles % 2 == 0 ? 2 : 0;
-}
-
-int launch_stream(const GemmArgs& g, int m_tiles, int tiles, int ctas, int share, cudaStream_t st) {
+int launch_stream(const GemmArgs& g, int m_tiles, int tiles, int ctas, cudaStream_t st) {
     switch (output_fmt(g.out)) {
-        case FMT_FF: return launch_emb<FMT_FF>(g, m_tiles, tiles, ctas, share, st);
-        case FMT_C128: return launch_emb<FMT_C128>(g, m_tiles, tiles, ctas, share, st);
-        default: return launch_emb<FMT_C64>(g, m_tiles, tiles, ctas, share, st);
+        case FMT_FF: return launch_emb<FMT_FF>(g, m_tiles, tiles, ctas, st);
+        case FMT_C128: return launch_emb<FMT_C128>(g, m_tiles, tiles, ctas, st);
+        default: return launch_emb<FMT_C64>(g, m_tiles, tiles, ctas, st);
     }
 }
 

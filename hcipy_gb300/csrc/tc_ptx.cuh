@@ -70,16 +70,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
-// The same box into the same place of every CTA of the cluster in `mask`, whose barriers at that place each count it.
-__device__ __forceinline__ void tma_load_3d_multicast(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                                      uint32_t bar, uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%2, "
-        "%3, %4}], [%5], %6;" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar), "h"(mask)
-        : "memory");
-}
-
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
                  : "memory");
@@ -132,14 +122,6 @@ __device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t alo, uint3
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
-}
-
-// The same arrival on the barrier at the same place of every CTA of the cluster in `mask`.
-__device__ __forceinline__ void umma_commit_multicast(uint32_t bar, uint16_t mask) {
-    asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-        "h"(mask)
-        : "memory");
 }
 
 // 32 lanes x 32 bits, 16 consecutive columns: thread i of the warp gets lane (base lane + i).
