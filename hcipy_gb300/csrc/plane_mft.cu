@@ -2,11 +2,16 @@
 // that cut fields into planes, and the two GEMMs of a transform (plane_gemm.cuh describes the arithmetic).
 //
 // A transform out = alpha L . in . R (in K1 x K2, R K2 x C, L R x K1) runs as
-//   1. rows of in -> planes (K2 long)
+//   1. rows of in, times the source weights along them -> planes (K2 long)
 //   2. T^T[c][k1] = sum_k2 in[k1, k2] R[k2, c]          (GEMM over K2, written transposed)
-//   3. rows of T^T -> planes (K1 long)
+//   3. rows of T^T, times the source weights along them -> planes (K1 long)
 //   4. out[r][c] = alpha sum_k1 T^T[c][k1] L[r, k1]     (GEMM over K1, written transposed, with the epilogue)
 // for every direction, the fields of a batch stacked along the rows of both GEMMs.
+//
+// The planes keep their bits below a row's maximum, so what varies along the sum belongs into one operand: the weights of
+// a non-uniform source grid multiply the field before it is cut, and the constants are phases of modulus 1.  With the
+// weights in the constants, weights over 9 decades (a logarithmic axis) against a field that falls as they rise lost
+// all but 12 bits of complex64 and 28 of complex128.
 #include "plane_mft.cuh"
 #include "plane_gemm.cuh"
 
@@ -137,15 +142,27 @@ __device__ __forceinline__ void load4(const double2* p, int k0, int K, double* r
 // One CTA per row of K complex values: the row's scale, and its planes [Re | Im], each Kp long with zeros past K.
 // Four values per thread and step, kept in registers between the maximum and the cut up to G steps (a longer row is
 // read twice), so the pass is bound by the bytes it moves: 8 B in and 8 B out per complex64 value, 16 and 28 B per
-// complex128 value.
-template <typename T, int G>
+// complex128 value.  W: value k of a row is multiplied by wk[k].
+template <typename T, int G, bool W>
 __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>::type* __restrict__ in, long long ld,
-                                                         int K, int Kp, __half* __restrict__ planes,
-                                                         long long plane_stride, int kpitch,
+                                                         int K, int Kp, const T* __restrict__ wk,
+                                                         __half* __restrict__ planes, long long plane_stride,
+                                                         int kpitch,
                                                          typename Shape<T>::Scale* __restrict__ scale_out) {
     using MB = MaxBits<T>;
     constexpr int NP = Shape<T>::NP;
     __shared__ typename MB::V red[8];
+    auto load = [&](const typename cplx<T>::type* p, int k0, T* a, T* b) {
+        load4(p, k0, K, a, b);
+        if constexpr (W) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const T w = k0 + j < K ? __ldg(&wk[k0 + j]) : T(0);
+                a[j] *= w;
+                b[j] *= w;
+            }
+        }
+    };
     const long long m = blockIdx.x;
     const typename cplx<T>::type* row = in + m * ld;
     const int step = 4 * blockDim.x;
@@ -153,13 +170,13 @@ __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>:
     typename MB::V mx = 0;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        load4(row, 4 * threadIdx.x + g * step, K, re[g], im[g]);
+        load(row, 4 * threadIdx.x + g * step, re[g], im[g]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx = max(mx, max(MB::of(re[g][j]), MB::of(im[g][j])));
     }
     for (int k0 = 4 * threadIdx.x + G * step; k0 < K; k0 += step) {
         T a[4], b[4];
-        load4(row, k0, K, a, b);
+        load(row, k0, a, b);
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx = max(mx, max(MB::of(a[j]), MB::of(b[j])));
     }
@@ -184,28 +201,24 @@ __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>:
     }
     for (int k0 = 4 * threadIdx.x + G * step; k0 < Kp; k0 += step) {
         T a[4], b[4];
-        load4(row, k0, K, a, b);
+        load(row, k0, a, b);
         put(k0, a, b);
     }
 }
 
-// One CTA per column n of a constant operand V[n][k] = wn[n] wk[k] exp(sign i a[n] b[k]), evaluated in float64 as
-// the phase matrices of the CUDA-core form are: the rows [Re | -Im] and [Im | Re] of its embedding.
+// One CTA per column n of a constant operand V[n][k] = wn[n] exp(sign i a[n] b[k]), evaluated in float64 as the phase
+// matrices of the CUDA-core form are: the rows [Re | -Im] and [Im | Re] of its embedding.
 template <typename T>
 __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const double* __restrict__ a,
                                                           const double* __restrict__ b, double sign,
-                                                          const double* __restrict__ wn, const double* __restrict__ wk,
-                                                          __half* __restrict__ planes, long long plane_stride,
-                                                          int kpitch, typename Shape<T>::Scale* __restrict__ scale_out) {
+                                                          const double* __restrict__ wn, __half* __restrict__ planes,
+                                                          long long plane_stride, int kpitch,
+                                                          typename Shape<T>::Scale* __restrict__ scale_out) {
     using MB = MaxBits<T>;
     constexpr int NP = Shape<T>::NP;
-    __shared__ typename MB::V red[8];
     const int n = blockIdx.x;
-    const double w0 = wn ? wn[n] : 1.0;
-    // both parts are at most |w| (rounded up by nothing: cos and sin do not exceed 1)
-    typename MB::V mx = 0;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) mx = max(mx, MB::of((T)(w0 * (wk ? wk[k] : 1.0))));
-    const auto s = MB::scale(block_max(mx, red));
+    const double w = wn ? wn[n] : 1.0;
+    const auto s = MB::scale(MB::of((T)w));  // both parts are at most |w|
     if (threadIdx.x == 0) scale_out[n] = s;
     const auto f = cut_factor(s);
     const long long r_re = (long long)(n >> 3) * 16 + (n & 7), r_im = r_re + 8;
@@ -217,7 +230,6 @@ __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const d
             double sn = 0.0, co = 0.0;
             if (k < K) {
                 sincos(a[n] * b[k], &sn, &co);
-                const double w = w0 * (wk ? wk[k] : 1.0);
                 co *= w;
                 sn *= w * sign;
             }
@@ -238,6 +250,11 @@ __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const d
             *reinterpret_cast<uint2*>(pl + r_im * kpitch + Kp + k0) = cr[p];
         }
     }
+}
+
+// Weights of a source axis in the fields' type.
+template <typename T> __global__ void plane_weights_kernel(int K, const double* __restrict__ w, T* __restrict__ out) {
+    for (int k = threadIdx.x; k < K; k += blockDim.x) out[k] = (T)w[k];
 }
 
 // ---- host side ----------------------------------------------------------------------------------------------
@@ -312,19 +329,20 @@ template <typename T> int encode_map(CUtensorMap* map, const PlaneMat& m, int bo
 }
 
 template <typename T>
-int launch_rows(const void* in, long long rows, int K, const PlaneMat& m, cudaStream_t st) {
+int launch_rows(const void* in, long long rows, int K, const void* wk, const PlaneMat& m, cudaStream_t st) {
     using Cx = typename cplx<T>::type;
     using Sc = typename Shape<T>::Scale;
     const int threads = std::min<int>(256, (int)round_up((m.Kp + 3) / 4, 32));
     const int steps = (m.Kp + 4 * threads - 1) / (4 * threads);
     const unsigned grid = (unsigned)rows;
-    auto run = [&](auto g) {
-        plane_rows_kernel<T, decltype(g)::value><<<grid, threads, 0, st>>>((const Cx*)in, K, K, m.Kp, m.planes,
-                                                                          m.plane_stride(), m.kpitch, (Sc*)m.scale);
+    auto run = [&](auto g, auto weighted) {
+        plane_rows_kernel<T, decltype(g)::value, decltype(weighted)::value><<<grid, threads, 0, st>>>(
+            (const Cx*)in, K, K, m.Kp, (const T*)wk, m.planes, m.plane_stride(), m.kpitch, (Sc*)m.scale);
     };
-    if (steps == 1) run(std::integral_constant<int, 1>());
-    else if (steps == 2) run(std::integral_constant<int, 2>());
-    else run(std::integral_constant<int, 4>());
+    if (wk) run(std::integral_constant<int, 1>(), std::true_type());
+    else if (steps == 1) run(std::integral_constant<int, 1>(), std::false_type());
+    else if (steps == 2) run(std::integral_constant<int, 2>(), std::false_type());
+    else run(std::integral_constant<int, 4>(), std::false_type());
     return launch_status("plane_rows_kernel");
 }
 
@@ -416,6 +434,8 @@ struct PlaneMft {
     int dtype, nx, ny, nu, nv;
     void* mem = nullptr;
     PlaneMat rgt[3], lft[3];  // by direction: the operand along x (R) and the one along y (L)
+    void* wk2[3] = {};        // weights along the rows of the field (K2 of them) and of T^T (K1), or nullptr
+    void* wk1[3] = {};
     int* status = nullptr;
 };
 
@@ -477,10 +497,10 @@ template <typename T> bool takes(const Dims& d, int batch) {
 }
 
 template <typename T> int make_const(PlaneMat& m, int N, const double* a, const double* b, double sign,
-                                     const double* wn, const double* wk, cudaStream_t st) {
+                                     const double* wn, cudaStream_t st) {
     m.n = N;
     HX_TRY(encode_map<T>(&m.map, m, Shape<T>::BN));
-    plane_const_kernel<T><<<(unsigned)N, 256, 0, st>>>(m.K, m.Kp, a, b, sign, wn, wk, m.planes, m.plane_stride(),
+    plane_const_kernel<T><<<(unsigned)N, 256, 0, st>>>(m.K, m.Kp, a, b, sign, wn, m.planes, m.plane_stride(),
                                                        m.kpitch, (typename Shape<T>::Scale*)m.scale);
     return launch_status("plane_const_kernel");
 }
@@ -495,6 +515,11 @@ int create_t(PlaneMft* p, const double* x, const double* y, const double* u, con
             carve_mat<T>(c, p->rgt[d], 2 * round_up(q.C, 8), q.C, q.K2);
             carve_mat<T>(c, p->lft[d], 2 * round_up(q.R, 8), q.R, q.K1);
         }
+        auto weights = [&](const double* w, int n) { return w ? c.take(sizeof(T) * (size_t)n) : nullptr; };
+        p->wk2[HX_FORWARD] = weights(wx, p->nx);
+        p->wk1[HX_FORWARD] = weights(wy, p->ny);
+        p->wk2[HX_BACKWARD] = weights(wu, p->nu);
+        p->wk1[HX_BACKWARD] = weights(wv, p->nv);
         p->status = (int*)c.take(sizeof(int));
     };
     Carver count(nullptr);
@@ -503,13 +528,22 @@ int create_t(PlaneMft* p, const double* x, const double* y, const double* u, con
     HX_TRY(cuda_status(cudaMemsetAsync(p->mem, 0, count.off, st), "memset plane MFT plan"));
     Carver c(p->mem);
     layout(c);
-    HX_TRY(make_const<T>(p->rgt[HX_FORWARD], p->nu, u, x, -1.0, nullptr, wx, st));
-    HX_TRY(make_const<T>(p->lft[HX_FORWARD], p->nv, v, y, -1.0, nullptr, wy, st));
-    HX_TRY(make_const<T>(p->rgt[HX_BACKWARD], p->nx, x, u, +1.0, nullptr, wu, st));
-    HX_TRY(make_const<T>(p->lft[HX_BACKWARD], p->ny, y, v, +1.0, nullptr, wv, st));
+    HX_TRY(make_const<T>(p->rgt[HX_FORWARD], p->nu, u, x, -1.0, nullptr, st));
+    HX_TRY(make_const<T>(p->lft[HX_FORWARD], p->nv, v, y, -1.0, nullptr, st));
+    HX_TRY(make_const<T>(p->rgt[HX_BACKWARD], p->nx, x, u, +1.0, nullptr, st));
+    HX_TRY(make_const<T>(p->lft[HX_BACKWARD], p->ny, y, v, +1.0, nullptr, st));
+    auto weights = [&](void* out, int n, const double* w) {
+        if (!out) return (int)HX_OK;
+        plane_weights_kernel<T><<<1, 256, 0, st>>>(n, w, (T*)out);
+        return launch_status("plane_weights_kernel");
+    };
+    HX_TRY(weights(p->wk2[HX_FORWARD], p->nx, wx));
+    HX_TRY(weights(p->wk1[HX_FORWARD], p->ny, wy));
+    HX_TRY(weights(p->wk2[HX_BACKWARD], p->nu, wu));
+    HX_TRY(weights(p->wk1[HX_BACKWARD], p->nv, wv));
     if (own_adjoint) {
-        HX_TRY(make_const<T>(p->rgt[HX_ADJOINT], p->nx, x, u, +1.0, wx, nullptr, st));
-        HX_TRY(make_const<T>(p->lft[HX_ADJOINT], p->ny, y, v, +1.0, wy, nullptr, st));
+        HX_TRY(make_const<T>(p->rgt[HX_ADJOINT], p->nx, x, u, +1.0, wx, st));
+        HX_TRY(make_const<T>(p->lft[HX_ADJOINT], p->ny, y, v, +1.0, wy, st));
     } else {
         p->rgt[HX_ADJOINT] = p->rgt[HX_BACKWARD];
         p->lft[HX_ADJOINT] = p->lft[HX_BACKWARD];
@@ -529,7 +563,7 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
         carve_pass<T>(ws, d, nb, &q);
         const Cx* src_f = (const Cx*)in + (long long)b0 * d.K1 * d.K2;
         const long long oplane = (long long)d.R * d.C;
-        HX_TRY(launch_rows<T>(src_f, (long long)nb * d.K1, d.K2, q.s1, st));
+        HX_TRY(launch_rows<T>(src_f, (long long)nb * d.K1, d.K2, p->wk2[direction], q.s1, st));
         PlaneArgs<T> g1;
         memset(&g1, 0, sizeof(g1));
         g1.rows_per_field = d.K1;
@@ -541,7 +575,7 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
         g1.parts = (typename Shape<T>::Acc*)q.parts;
         g1.status = p->status;
         HX_TRY(launch_gemm<T>(g1, q.s1, p->rgt[direction], throughput, (double)nb * d.K1 * d.K2 * d.C, st));
-        HX_TRY(launch_rows<T>(q.t, (long long)nb * d.C, d.K1, q.s2, st));
+        HX_TRY(launch_rows<T>(q.t, (long long)nb * d.C, d.K1, p->wk1[direction], q.s2, st));
         PlaneArgs<T> g2;
         memset(&g2, 0, sizeof(g2));
         g2.rows_per_field = d.C;
