@@ -5,40 +5,40 @@
 // warp (consecutive m) store consecutive addresses straight from the accumulators, and so that the second GEMM of a
 // transform reads the first one's result by contiguous rows.
 //
-// Operands.  Every row of A and of B is scaled by a power of two and cut into fp16 planes:
-//   complex64 : two planes, x = s (h + l), h and l the fp16 roundings of x / s and of x / s - h, which keeps 22 bits
-//               of every element; the products h l, l h and h h go to one FP32 accumulator, the small ones first.
-//   complex128: seven planes of balanced base-256 digits, x = s sum_i d_i 2^(-7 - 8 i) with d_i in [-128, 128],
-//               55 bits below the row maximum; the 28 products d_i d_j with i + j <= 6 go to seven accumulators, one
-//               per level i + j.
+// Operands.  Every row of A and of B is scaled by a power of two and cut into fp16 planes of balanced digits,
+// x = 2^E sum_i d_i w_i with |x| <= 2^E:
+//   complex64 : three digits of base 512, d_i in [-256, 256], w_i = 2^(-8 - 9 i), which leaves 2^-27 of 2^E at most;
+//               the six products d_i d_j with i + j <= 2 go to three accumulators, one per level i + j;
+//   complex128: seven digits of base 256, d_i in [-128, 128], w_i = 2^(-7 - 8 i), which leaves 2^-56; the 28 products
+//               with i + j <= 6 go to seven accumulators.
 // A holds [Ar | Ai] per row (K' = 2K), B holds the complex embedding in blocks of 8 complex columns: the 8 real
 // columns [Br | -Bi], then the 8 imaginary ones [Bi | Br].
 //
-// Sums.  The tensor cores truncate an FP32 sum that no longer fits 24 bits (a sum of 4096 positive
-// products comes out 2.5e-5 low, of 64 products 1.5e-7 low: measured against float64), so no accumulator runs long:
-//   complex64 : 32 terms of K', then the accumulator is added to FP32 registers in round-to-nearest, in blocks of 16
-//               partial sums.  Such a sum is truncated after its first 16 terms and at the end, by half an ulp on
-//               average: 2^-24 / (2 ln 2) = 4.3e-8 of a value with mantissas spread over their logarithm, and half of
-//               that for the first truncation, 6.4e-8 together (6.5e-8 measured), whatever the signs of the terms.
-//               A factor so close to 1 on every GEMM adds up along a chain of transforms, so it is taken back on
-//               average (Sums<float>::add);
-//   complex128: 128 terms: every level is then an integer below 7 * 128 * 2^14 < 2^24, hence exact, and is added to
-//               64-bit integers (levels 0-3 in one, 4-6 in another), exact over any K the plans take.
-// The error of a complex128 transform is that of its operands (2^-56 of a row maximum) and of the dropped products
-// (below 2^-56 of the two scales), both under the rounding of a float64 product.
+// Sums.  The tensor cores truncate an FP32 sum that no longer fits 24 bits (a sum of 4096 positive products comes out
+// 2.5e-5 low, of 64 products 1.5e-7 low: measured against float64), so the accumulators hold whole numbers that fit:
+//   complex64 : 256 terms of K': level 0 is at most 256 * 2^16 = 2^24, hence exact, and is added to 32-bit integers (2^30
+//               over the longest K' of 16384).  Levels 1 and 2 weigh 2^-9 and 2^-18 of it: what they lose below 24 bits is
+//               below 2^-32 of the terms' size.  They are added in FP32, and the sum is rounded once, at the end.
+//   complex128: 128 terms: every level is below 7 * 128 * 2^14 < 2^24, hence exact, and is added to 64-bit integers
+//               (levels 0-3 in one, 4-6 in another), exact over any K the plans take.
+// The error of a transform is that of its operands (above), of the dropped products (digits 1 and 2 in complex64: 2^-26 of the
+// two scales at most) and one rounding of each sum: 3.5-7.5e-8 for complex64, 1e-7 for gradients through six transforms.
+// Two planes of floating fp16 values with three products, 22 bits and FP32 sums of 32 terms were a quarter faster (Lyot
+// pass below 333 us), but what the truncated sums lost (6e-8 of their value on average) added up along a chain: such
+// gradients came out 3.6-5.3e-7 off where the CUDA cores give 2.6-3.5e-7, and a field of one pixel 1.0-2.2e-7 where they
+// give 0.4-0.6e-7.
 //
 // Pipeline.  One CTA per 128 rows x BN real columns (BN = 128 for complex64, 64 for complex128, whose seven levels
 // take 448 of the 512 TMEM columns): warp 0 issues TMA boxes of all planes of a K step, warp 1 the MMAs, the others
-// drain.  Each accumulator has its own pair of barriers, so level l of the next partial sum starts as soon as level
-// l of this one is drained: complex64 alternates two sets of accumulators, complex128 drains its levels in the order
-// in which the next step's MMAs reach them.
+// drain.  Each level has its own pair of barriers, so level l of the next partial sum starts as soon as level l of this
+// one is drained, in the order in which the next step's MMAs reach them.
 // With few tiles the CTAs of a thread-block cluster split K and add their partial sums in rank order, each CTA
 // finishing a slice of the columns.  The sums travel through L2 under the cluster's barrier: through distributed shared
 // memory they moved at 7 to 13 bytes per clock and SM.
 // Measured against the GEMMs on the CUDA cores: a complex128 lens of 512^2 points to 256^2 1060 -> 72 us (float64 pipe), a
-// complex64 Lyot pass over four fields of 1024^2 points 1700 -> 333 us (FP32 pipe).  complex64 is bound by shared memory
-// (1270 clocks per 64 K', of which its MMAs take 768), complex128 by the epilogue (10 of 38 thousand clocks are MMAs
-// where K is split eight ways).
+// complex64 Lyot pass over four fields of 1024^2 points 1700 -> 431 us (FP32 pipe).  complex64 is bound by shared memory (per
+// 16 K' its MMAs read 40 KB in 384 clocks while the loads write 24 KB, and it moves 128 bytes a clock), complex128 by the
+// epilogue (10 of 38 thousand clocks are MMAs where K is split eight ways).
 // All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word.
 #pragma once
 
@@ -52,19 +52,21 @@ namespace pg {
 
 constexpr int BM = 128;            // rows of A per tile (TMEM lanes)
 constexpr uint64_t WAIT_LIMIT = 2000000000ull;
-constexpr int NAN_EXP = -(1 << 28);  // row exponent of a row that holds an infinity or a NaN (complex128)
+constexpr int NAN_EXP = -(1 << 28);  // exponent of a row that holds an infinity or a NaN
 
-// Planes (NP), accumulators (LV), real columns per tile (BN), K' per stage (BK), accumulator sets (SETS), stages per
-// partial sum (CT) and partial sums per stage (PPS), pipeline stages (ST), epilogue threads (EPI: complex64 drains often
-// and little, complex128 seldom and much, and its conversions want warps).
+// Planes (NP), levels (LV), real columns per tile (BN), K' per stage (BK), stages per partial sum (CT), pipeline stages
+// (ST), epilogue threads (EPI: the conversions at the end want warps).
 template <typename T> struct Shape;
 template <> struct Shape<float> {
-    static constexpr int NP = 2, LV = 1, BN = 128, BK = 64, SETS = 4, CT = 1, PPS = 2, ST = 3, EPI = 256;
-    using Acc = float;
-    using Scale = float;
+    static constexpr int NP = 3, LV = 3, BN = 128, BK = 32, CT = 8, ST = 4, EPI = 512;
+    struct __align__(8) Acc {
+        int hi;    // value = hi 2^-16 + lo 2^-34 (times the scales)
+        float lo;
+    };
+    using Scale = int;  // exponent of the power-of-two scale
 };
 template <> struct Shape<double> {
-    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, SETS = 1, CT = 4, PPS = 1, ST = 2, EPI = 512;
+    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, CT = 4, ST = 2, EPI = 512;
     struct __align__(16) Acc {
         long long hi, lo;  // value = hi 2^-38 + lo 2^-62 (times the scales)
     };
@@ -83,9 +85,8 @@ template <typename T> struct Layout {
     static constexpr int THREADS = S::EPI + 64;     // TMA warp, MMA warp, epilogue warps
     static constexpr int COLS = S::BN / (S::EPI / BM);  // real columns per epilogue thread
     static constexpr int LD = COLS < 32 ? COLS : 32;    // columns per TMEM load
-    static constexpr int NACC = S::SETS * S::LV;
     static constexpr int TMEM_COLS = 512;
-    static_assert(NACC * S::BN <= TMEM_COLS, "the accumulators must fit TMEM");
+    static_assert(S::LV * S::BN <= TMEM_COLS, "the accumulators must fit TMEM");
     static_assert(BM * S::BN * (int)sizeof(typename S::Acc) <= PIPE, "partial sums must fit the pipeline buffers");
     static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
 };
@@ -166,29 +167,47 @@ __device__ __noinline__ double scaled_value(long long hi, long long lo, int e) {
     return scalbn(fma((double)hi, 0x1p24, (double)lo), e);
 }
 
-__device__ __forceinline__ float acc_value(const float& a, float rs, float cs, bool&) { return a * cs * rs; }
+// (hi 2^18 + lo) 2^e with one rounding to 24 bits (and, where the result is subnormal, one more).
+__device__ __forceinline__ float fixed_to_float(int hi, float lo, int e) {
+    const float f = (float)hi;
+    const float v = fmaf(f, 0x1p18f, fmaf((float)(hi - (int)f), 0x1p18f, lo));
+    const int c = min(max(e, -252), 254), h = c >> 1;  // past these v 2^e is 0 or infinite either way
+    return v * __int_as_float((h + 127) << 23) * __int_as_float((c - h + 127) << 23);
+}
+
+__device__ __forceinline__ float acc_value(const Shape<float>::Acc& a, int re, int ce, bool& rare) {
+    rare |= re == NAN_EXP || ce == NAN_EXP;
+    return fixed_to_float(a.hi, a.lo, re + ce - 34);
+}
 __device__ __forceinline__ double acc_value(const Shape<double>::Acc& a, int re, int ce, bool& rare) {
     rare |= re == NAN_EXP || ce == NAN_EXP;
     return fixed_to_double(a.hi, a.lo, re + ce - 62, rare);
 }
-__device__ __forceinline__ float acc_rare(const float& a, float rs, float cs) { return a * cs * rs; }
+__device__ __forceinline__ float acc_rare(const Shape<float>::Acc& a, int re, int ce) {
+    if (re == NAN_EXP || ce == NAN_EXP) return __int_as_float(0x7fc00000);
+    return fixed_to_float(a.hi, a.lo, re + ce - 34);
+}
 __device__ __forceinline__ double acc_rare(const Shape<double>::Acc& a, int re, int ce) {
     if (re == NAN_EXP || ce == NAN_EXP) return __longlong_as_double(0x7ff8000000000000ll);
     return scaled_value(a.hi, a.lo, re + ce - 62);
 }
 
-__device__ __forceinline__ void acc_add(float& a, const float& b) { a += b; }
-__device__ __forceinline__ void acc_add(Shape<double>::Acc& a, const Shape<double>::Acc& b) {
+template <typename A> __device__ __forceinline__ void acc_add(A& a, const A& b) {
     a.hi += b.hi;
     a.lo += b.lo;
 }
 
 // Partial sums of the other CTAs of a K split travel through L2.
-__device__ __forceinline__ void put_part(float* p, float v) { __stcg(p, v); }
+__device__ __forceinline__ void put_part(Shape<float>::Acc* p, const Shape<float>::Acc& v) {
+    __stcg(reinterpret_cast<int2*>(p), make_int2(v.hi, __float_as_int(v.lo)));
+}
 __device__ __forceinline__ void put_part(Shape<double>::Acc* p, const Shape<double>::Acc& v) {
     __stcg(reinterpret_cast<longlong2*>(p), make_longlong2(v.hi, v.lo));
 }
-__device__ __forceinline__ float get_part(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ Shape<float>::Acc get_part(const Shape<float>::Acc* p) {
+    const int2 v = __ldcg(reinterpret_cast<const int2*>(p));
+    return {v.x, __int_as_float(v.y)};
+}
 __device__ __forceinline__ Shape<double>::Acc get_part(const Shape<double>::Acc* p) {
     const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(p));
     return {v.x, v.y};
@@ -198,28 +217,21 @@ __device__ __forceinline__ Shape<double>::Acc get_part(const Shape<double>::Acc*
 template <typename T> struct Sums;
 template <> struct Sums<float> {
     static constexpr int COLS = Layout<float>::COLS;
-    float tot[COLS], blk[COLS];
-    int n = 0;
+    Shape<float>::Acc a[COLS];
     __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) tot[j] = blk[j] = 0.0f;
+        for (int j = 0; j < COLS; ++j) a[j] = {0, 0.0f};
     }
-    // Every second partial sum times 1 + 2^-23, in the one rounding of the addition: 6.0e-8 of the 6.4e-8 that the
-    // truncated sums lose on average (see above).
+    // level 0 in units of its own, levels 1 and 2 (2^9 and 1) in units of level 2
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
-        const float w = (n & 1) ? 1.0f : 1.0f + 0x1p-23f;
 #pragma unroll
-        for (int j = 0; j < Layout<float>::LD; ++j) blk[j0 + j] = fmaf(v[j], w, blk[j0 + j]);
-    }
-    __device__ __forceinline__ void end_partial(bool last) {
-        if ((++n & 15) != 0 && !last) return;
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) {
-            tot[j] += blk[j];
-            blk[j] = 0.0f;
+        for (int j = 0; j < Layout<float>::LD; ++j) {
+            if (L == 0) a[j0 + j].hi += __float2int_rn(v[j]);
+            else if (L == 1) a[j0 + j].lo = fmaf(v[j], 512.0f, a[j0 + j].lo);
+            else a[j0 + j].lo += v[j];
         }
     }
-    __device__ __forceinline__ float get(int j) const { return tot[j]; }
+    __device__ __forceinline__ const Shape<float>::Acc& get(int j) const { return a[j]; }
 };
 template <> struct Sums<double> {
     static constexpr int COLS = Layout<double>::COLS;
@@ -238,9 +250,16 @@ template <> struct Sums<double> {
             else a[j0 + j].lo += p;
         }
     }
-    __device__ __forceinline__ void end_partial(bool) {}
     __device__ __forceinline__ const Shape<double>::Acc& get(int j) const { return a[j]; }
 };
+
+// f with the compile-time numbers 0 .. N - 1.
+template <int N, typename F> __device__ __forceinline__ void each_level(F&& f) {
+    if constexpr (N > 0) {
+        each_level<N - 1>(f);
+        f(std::integral_constant<int, N - 1>());
+    }
+}
 
 // The finished columns of a tile: all of them, or with a K split over KS CTAs the ks-th of KS slices of its complex
 // columns, the CTA's own partial sums from shared memory and the others' from `others` (L2), added in rank order.
@@ -254,7 +273,7 @@ __device__ __forceinline__ void finish_columns(const PlaneArgs<T>& g, const type
     using Cx = typename cplx<T>::type;
     using Acc = typename Shape<T>::Acc;
     constexpr int TN = Layout<T>::TN, STEP = Shape<T>::EPI / BM, TNS = TN / KS;
-    constexpr int U = TNS / STEP < (sizeof(T) == 4 ? 4 : 2) ? TNS / STEP : (sizeof(T) == 4 ? 4 : 2);
+    constexpr int UMAX = sizeof(T) == 4 && KS < 4 ? 4 : 2, U = TNS / STEP < UMAX ? TNS / STEP : UMAX;
     static_assert(TNS % (STEP * U) == 0, "whole batches");
     constexpr int PART = TN * 2 * BM;  // one CTA's partial sums
     const int r = et & (BM - 1), m = m0 + r;
@@ -343,7 +362,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     const uint32_t raw = ptx::smem_addr(pg_smem);
     uint8_t* smem = pg_smem + ((1024 - (raw & 1023)) & 1023);
     uint8_t* extra = smem + LY::PIPE;
-    // full[ST], empty[ST], ready[NACC], drained[NACC], done
+    // full[ST], empty[ST], ready[LV], drained[LV], done
     uint64_t* bars = reinterpret_cast<uint64_t*>(extra);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra + 256);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(extra + 260);
@@ -352,9 +371,9 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     auto bar_full = [&](int s) { return ptx::smem_addr(&bars[s]); };
     auto bar_empty = [&](int s) { return ptx::smem_addr(&bars[S::ST + s]); };
     auto bar_ready = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + a]); };
-    auto bar_drained = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + LY::NACC + a]); };
-    const uint32_t bar_done = ptx::smem_addr(&bars[2 * S::ST + 2 * LY::NACC]);
-    static_assert((2 * S::ST + 2 * LY::NACC + 1) * 8 <= 256, "barriers");
+    auto bar_drained = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + S::LV + a]); };
+    const uint32_t bar_done = ptx::smem_addr(&bars[2 * S::ST + 2 * S::LV]);
+    static_assert((2 * S::ST + 2 * S::LV + 1) * 8 <= 256, "barriers");
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform
     const int KS = g.ksplit;
@@ -371,7 +390,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
             ptx::mbar_init(bar_full(s), 1);
             ptx::mbar_init(bar_empty(s), 1);
         }
-        for (int a = 0; a < LY::NACC; ++a) {
+        for (int a = 0; a < S::LV; ++a) {
             ptx::mbar_init(bar_ready(a), 1);
             ptx::mbar_init(bar_drained(a), S::EPI / 32);
         }
@@ -431,83 +450,56 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         bool ok = true;
         for (int i = 0; i < nkt && ok; ++i) {
             const int s = i % S::ST, u = i / S::ST;
-            const int part = i / S::CT * S::PPS, use = part / S::SETS;  // a stage's partial sums are of one use
-            const int set = part % S::SETS;
+            const int part = i / S::CT;
             const bool first = i % S::CT == 0, last = i % S::CT == S::CT - 1 || i == nkt - 1;
             ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, WAIT_LIMIT));
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t a0 = desc_lo(smem_a + s * LY::STAGE);
             const uint32_t b0 = a0 + (S::NP * LY::A_PLANE >> 4);
-            const uint32_t d0 = tmem + set * (S::LV * S::BN);
             constexpr uint32_t hi = desc_hi<LY::ROW_BYTES>();
             auto drained = [&](int l) {  // the accumulator's previous partial sum must have been read
                 if (ok)
-                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(set * S::LV + l), (use - 1) & 1,
-                                                                        WAIT_LIMIT));
+                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(l), (part - 1) & 1, WAIT_LIMIT));
                 ptx::tc_fence_after();
             };
             // planes pb .. pb + count - 1 of B, which follow one another as the levels do in TMEM
             auto mma = [&](auto count, int pa, int pb, int l, int kk, bool start) {
                 constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, S::BN * decltype(count)::value);
                 if (leader)
-                    ptx::umma_f16_lo(d0 + l * S::BN, a0 + ((pa * LY::A_PLANE + kk * 32) >> 4),
+                    ptx::umma_f16_lo(tmem + l * S::BN, a0 + ((pa * LY::A_PLANE + kk * 32) >> 4),
                                      b0 + ((pb * LY::B_PLANE + kk * 32) >> 4), hi, idesc, start);
             };
             using one = std::integral_constant<int, 1>;
-            if constexpr (S::LV == 1) {
-                // one accumulator: the small products h l and l h first, while the sum is small and is truncated little
-                static_assert(S::CT == 1 && S::SETS % S::PPS == 0, "whole partial sums per stage");
-                constexpr int KH = S::BK / 16 / S::PPS;
+            // The first step of a partial sum takes a level at a time, as the accumulators are read out.  The others
+            // take a plane of A at a time, against as many planes of B in one MMA as 256 columns hold: an MMA of 64
+            // columns reads 4 KB of A and 2 KB of B in its 32 clocks, more than shared memory gives beside the
+            // loads.  complex128: 10 MMAs and 96 KB per 16 K' instead of 28 and 168 KB, complex64: 4 and 40 KB instead
+            // of 6 and 48 KB.  Exact sums may be taken in any order.
+            constexpr int G = 256 / S::BN;
+            auto row = [&](auto plane, int kk) {
+                constexpr int P = decltype(plane)::value, CNT = S::LV - P;
+                mma(std::integral_constant<int, (CNT < G ? CNT : G)>{}, P, 0, P, kk, false);
+                if constexpr (CNT > G) mma(std::integral_constant<int, CNT - G>{}, P, G, P + G, kk, false);
+            };
+            static_assert(S::LV <= 2 * G, "two MMAs at most for each plane of A");
 #pragma unroll
-                for (int h = 0; h < S::PPS; ++h) {
-                    if (use > 0) drained(h);
+            for (int kk = 0; kk < S::BK / 16; ++kk) {
+                const bool end = kk == S::BK / 16 - 1 && last;
+                if (kk == 0 && first) {
 #pragma unroll
-                    for (int kk = h * KH; kk < (h + 1) * KH; ++kk) {
-                        mma(one{}, 0, 1, h, kk, kk == h * KH);
-                        mma(one{}, 1, 0, h, kk, false);
+                    for (int l = 0; l < S::LV; ++l) {
+                        if (part > 0) drained(l);
+#pragma unroll
+                        for (int p = 0; p <= l; ++p) mma(one{}, p, l - p, l, kk, p == 0);
+                        if (end && leader) ptx::umma_commit(bar_ready(l));
                     }
-#pragma unroll
-                    for (int kk = h * KH; kk < (h + 1) * KH; ++kk) mma(one{}, 0, 0, h, kk, false);
-                    if (leader) ptx::umma_commit(bar_ready(set + h));
-                }
-            } else {
-                // The first step of a partial sum takes a level at a time, as the accumulators are read out.  The others
-                // take a plane of A at a time, against up to four planes of B (256 columns) in one MMA: an MMA of 64
-                // columns reads 4 KB of A and 2 KB of B in its 32 clocks, more than shared memory gives beside the
-                // loads.  10 MMAs and 96 KB per 16 K' instead of 28 and 168 KB; the sums are whole numbers, exact in
-                // any order.
-                constexpr int G = 256 / S::BN;
-                auto row = [&](auto plane, int kk) {
-                    constexpr int P = decltype(plane)::value, CNT = S::LV - P;
-                    mma(std::integral_constant<int, (CNT < G ? CNT : G)>{}, P, 0, P, kk, false);
-                    if constexpr (CNT > G) mma(std::integral_constant<int, CNT - G>{}, P, G, P + G, kk, false);
-                };
-                static_assert(S::LV == 7 && S::LV <= 2 * G, "the planes listed below, two MMAs for each at most");
-#pragma unroll
-                for (int kk = 0; kk < S::BK / 16; ++kk) {
-                    const bool end = kk == S::BK / 16 - 1 && last;
-                    if (kk == 0 && first) {
-#pragma unroll
-                        for (int l = 0; l < S::LV; ++l) {
-                            if (use > 0) drained(l);
-#pragma unroll
-                            for (int p = 0; p <= l; ++p) mma(one{}, p, l - p, l, kk, p == 0);
-                            if (end && leader) ptx::umma_commit(bar_ready(set * S::LV + l));
-                        }
-                    } else {
-                        auto plane = [&](auto p) {  // with it the level of its own index has all its products
-                            row(p, kk);
-                            if (end && leader) ptx::umma_commit(bar_ready(set * S::LV + decltype(p)::value));
-                        };
-                        plane(std::integral_constant<int, 0>());
-                        plane(std::integral_constant<int, 1>());
-                        plane(std::integral_constant<int, 2>());
-                        plane(std::integral_constant<int, 3>());
-                        plane(std::integral_constant<int, 4>());
-                        plane(std::integral_constant<int, 5>());
-                        plane(std::integral_constant<int, 6>());
-                    }
+                } else {
+                    auto plane = [&](auto p) {  // with it the level of its own index has all its products
+                        row(p, kk);
+                        if (end && leader) ptx::umma_commit(bar_ready(decltype(p)::value));
+                    };
+                    each_level<S::LV>(plane);
                 }
             }
             if (leader) ptx::umma_commit(bar_empty(s));
@@ -531,14 +523,12 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         Sums<T> sums;
         sums.clear();
         bool live = true;
-        const int nparts = (nkt + S::CT - 1) / S::CT * S::PPS;
+        const int nparts = (nkt + S::CT - 1) / S::CT;
 #pragma unroll 1
         for (int p = 0; p < nparts; ++p) {
-            const int set = p % S::SETS, ph = (p / S::SETS) & 1;
             auto level = [&](auto lc) {
                 constexpr int l = decltype(lc)::value;
-                const int a = set * S::LV + l;
-                if (live && !ptx::mbar_wait_bounded(bar_ready(a), ph, WAIT_LIMIT)) give_up();
+                if (live && !ptx::mbar_wait_bounded(bar_ready(l), p & 1, WAIT_LIMIT)) give_up();
                 // warp-uniform: the TMEM loads are .sync.aligned
                 live = __shfl_sync(0xffffffffu, (int)(live && *abort_flag == 0), 0) != 0;
                 if (!live) return;
@@ -546,24 +536,15 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
 #pragma unroll
                 for (int j0 = 0; j0 < COLS; j0 += LY::LD) {
                     float v[LY::LD];
-                    tmem_ld<LY::LD>(tmem + lane_base + a * S::BN + slice * COLS + j0, v);
+                    tmem_ld<LY::LD>(tmem + lane_base + l * S::BN + slice * COLS + j0, v);
                     sums.template add<l>(j0, v);
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar_drained(a));
+                if (lane == 0) ptx::mbar_arrive(bar_drained(l));
             };
-            level(std::integral_constant<int, 0>());
-            if constexpr (S::LV > 1) {
-                level(std::integral_constant<int, 1>());
-                level(std::integral_constant<int, 2>());
-                level(std::integral_constant<int, 3>());
-                level(std::integral_constant<int, 4>());
-                level(std::integral_constant<int, 5>());
-                level(std::integral_constant<int, 6>());
-            }
+            each_level<S::LV>(level);
             if (!live) break;
-            sums.end_partial(p == nparts - 1);
         }
         // every warp has seen the last accumulators, so this CTA's copies and MMAs are complete
         ptx::named_barrier(1, S::EPI);

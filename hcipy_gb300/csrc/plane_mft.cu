@@ -26,22 +26,21 @@ namespace {
 
 // ---- cutting values into planes -----------------------------------------------------------------------------
 
-// Power of two s with |x| / s <= 2^15 for every |x| <= mx: the fp16 value h of x / s then leaves room for a second one
-// of the same weight, x / s - h, whose 11 bits are normal down to 2^-18 of the row's maximum.  s and 1 / s are normal
-// floats, and a row below 2^-111 keeps every bit of its subnormal values.
-__device__ __forceinline__ float plane_scale(float mx) {
-    if (!(mx > 0.0f)) return 1.0f;
-    int e = 128;  // infinities: the planes then hold infinities and NaNs
-    if (isfinite(mx)) frexpf(mx, &e);
-    return ldexpf(1.0f, max(e, -111) - 15);
-}
-
 // Exponent E with |x| <= 2^E for every |x| whose bit pattern is at most mx.
 __device__ __forceinline__ int plane_exponent(unsigned long long mx) {
     const int e = (int)(mx >> 52);
     if (e == 0x7ff) return NAN_EXP;
     if (mx == 0) return 0;
     return max(e - 1023 + ((mx & 0xfffffffffffffull) != 0), -1022);
+}
+
+// The same for a float's.
+__device__ __forceinline__ int plane_exponent(unsigned int mx) {
+    const int e = (int)(mx >> 23);
+    if (e == 0xff) return NAN_EXP;
+    if (mx == 0) return 0;
+    if (e == 0) return 32 - __clz((int)mx) - 149;
+    return e - 127 + ((mx & 0x7fffffu) != 0);
 }
 
 // x 2^(55 - E) rounded to an integer (|x| <= 2^E).
@@ -59,18 +58,29 @@ __device__ __forceinline__ long long to_fixed(double x, int E) {
     return (b >> 63) ? -(long long)q : (long long)q;
 }
 
-// The planes of four consecutive real values: out[p] holds them as four halves.
-__device__ __forceinline__ void cut4(const float* x, float inv, uint2* out) {
-    __half2 h[2], l[2];
+// The planes of four consecutive real values: out[p] holds them as four halves.  x 2^(26 - E) is an integer of 27 bits in
+// digits of 9 (two exact steps, since 2^(26 - E) itself may be out of range); with 256 added to each digit, bits 0-8
+// are plane 2, 9-17 plane 1 and what is left plane 0.
+__device__ __forceinline__ void cut4(const float* x, int E, uint2* out) {
+    const int k = E == NAN_EXP ? 0 : 26 - E, k1 = min(k, 120);
+    const float f1 = __int_as_float((k1 + 127) << 23), f2 = __int_as_float((k - k1 + 127) << 23);
+    uint32_t q[4];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const float a = x[2 * q] * inv, b = x[2 * q + 1] * inv;
-        h[q] = __floats2half2_rn(a, b);
-        const float2 f = __half22float2(h[q]);
-        l[q] = __floats2half2_rn(a - f.x, b - f.y);
+    for (int j = 0; j < 4; ++j) q[j] = (uint32_t)(E == NAN_EXP ? 0 : __float2int_rn(x[j] * f1 * f2)) + 0x4020100u;
+    const __half2 bias = __halves2half2(__ushort_as_half(0x6500), __ushort_as_half(0x6500));  // 1024 + 256
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        uint32_t w[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t a = p == 0 ? q[2 * i] >> 18 : (q[2 * i] >> (18 - 9 * p)) & 0x1ff;
+            const uint32_t b = p == 0 ? q[2 * i + 1] >> 18 : (q[2 * i + 1] >> (18 - 9 * p)) & 0x1ff;
+            const uint32_t u = 0x64006400u + (a | (b << 16));  // the halves 1024 + digit + 256
+            const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&u), bias);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        out[p] = make_uint2(w[0], w[1]);
     }
-    out[0] = make_uint2(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]));
-    out[1] = make_uint2(*reinterpret_cast<uint32_t*>(&l[0]), *reinterpret_cast<uint32_t*>(&l[1]));
 }
 
 __device__ __forceinline__ void cut4(const double* x, int E, uint2* out) {
@@ -99,15 +109,11 @@ template <typename T> struct MaxBits;
 template <> struct MaxBits<float> {
     using V = unsigned int;
     __device__ static V of(float x) { return __float_as_uint(x) & 0x7fffffffu; }
-    __device__ static float scale(V m) { return plane_scale(__uint_as_float(m > 0x7f800000u ? 0x7f800000u : m)); }
 };
 template <> struct MaxBits<double> {
     using V = unsigned long long;
     __device__ static V of(double x) { return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull; }
-    __device__ static int scale(V m) { return plane_exponent(m); }
 };
-__device__ __forceinline__ float cut_factor(float s) { return 1.0f / s; }
-__device__ __forceinline__ int cut_factor(int e) { return e; }
 
 template <typename V> __device__ __forceinline__ V block_max(V m, V* red) {
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -141,7 +147,7 @@ __device__ __forceinline__ void load4(const double2* p, int k0, int K, double* r
 
 // One CTA per row of K complex values: the row's scale, and its planes [Re | Im], each Kp long with zeros past K.
 // Four values per thread and step, kept in registers between the maximum and the cut up to G steps (a longer row is
-// read twice), so the pass is bound by the bytes it moves: 8 B in and 8 B out per complex64 value, 16 and 28 B per
+// read twice), so the pass is bound by the bytes it moves: 8 B in and 12 B out per complex64 value, 16 and 28 B per
 // complex128 value.  W: value k of a row is multiplied by wk[k].
 template <typename T, int G, bool W>
 __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>::type* __restrict__ in, long long ld,
@@ -180,9 +186,8 @@ __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>:
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx = max(mx, max(MB::of(a[j]), MB::of(b[j])));
     }
-    const auto s = MB::scale(block_max(mx, red));
-    if (threadIdx.x == 0) scale_out[m] = s;
-    const auto f = cut_factor(s);
+    const int f = plane_exponent(block_max(mx, red));
+    if (threadIdx.x == 0) scale_out[m] = f;
     auto put = [&](int k0, const T* a, const T* b) {
         uint2 cr[NP], ci[NP];
         cut4(a, f, cr);
@@ -218,9 +223,8 @@ __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const d
     constexpr int NP = Shape<T>::NP;
     const int n = blockIdx.x;
     const double w = wn ? wn[n] : 1.0;
-    const auto s = MB::scale(MB::of((T)w));  // both parts are at most |w|
-    if (threadIdx.x == 0) scale_out[n] = s;
-    const auto f = cut_factor(s);
+    const int f = plane_exponent(MB::of((T)w));  // both parts are at most |w|
+    if (threadIdx.x == 0) scale_out[n] = f;
     const long long r_re = (long long)(n >> 3) * 16 + (n & 7), r_im = r_re + 8;
     for (int k0 = 4 * threadIdx.x; k0 < Kp; k0 += 4 * blockDim.x) {
         T re[4], im[4], ni[4];
@@ -377,14 +381,13 @@ template <typename T> bool cluster_ok(int ks) {
     return cache[dev][ks] == 1;
 }
 
-// CTAs along K per tile: enough to occupy the SMs, each with at least one partial sum of complex128 (128 terms of K')
-// or four stages of complex64 (256 terms), below which the exchange costs more than the shorter chain saves.
+// CTAs along K per tile: enough to occupy the SMs, each with at least one partial sum (256 terms of K' in complex64, 128 in
+// complex128), below which the exchange costs more than the shorter chain saves.
 template <typename T> int k_split(long long tiles, int ktiles, bool throughput) {
     if (throughput) return 1;
     const int parts = (ktiles + Shape<T>::CT - 1) / Shape<T>::CT;
-    const int least = sizeof(T) == 4 ? 4 : 1;
     for (int ks : {8, 4, 2})
-        if (tiles * ks <= num_sms() && parts / ks >= least && cluster_ok<T>(ks)) return ks;
+        if (tiles * ks <= num_sms() && parts / ks >= 1 && cluster_ok<T>(ks)) return ks;
     return 1;
 }
 
