@@ -19,7 +19,8 @@ void set_error(const char* fmt, ...);
 void count_launch(int n = 1);
 
 // Host-side fault injection: when HX_FAULT names `site` ("alloc", "plan" or
-// "launch"), the entry point returns HX_ERR_INJECTED before touching the GPU.
+// "launch"), the entry point returns HX_ERR_INJECTED before touching the GPU.  "wait": the plain tensor-core GEMM runs with
+// a short limit on its waits and with a load left out, so that one of them runs out.
 bool fault_injected(const char* site);
 
 // Kernel timing (hx_trace_enable): a scope records a CUDA event on `stream` when it opens and another when it

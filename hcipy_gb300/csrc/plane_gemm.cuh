@@ -39,7 +39,8 @@
 // complex64 Lyot pass over four fields of 1024^2 points 1700 -> 431 us (FP32 pipe).  complex64 is bound by shared memory (per
 // 16 K' its MMAs read 40 KB in 384 clocks while the loads write 24 KB, and it moves 128 bytes a clock), complex128 by the
 // epilogue (10 of 38 thousand clocks are MMAs where K is split eight ways).
-// All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word.
+// All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word, and the CTA, with the
+// others of its cluster, writes NaN instead of sums that are not complete, so that no result looks like one.
 #pragma once
 
 #include "hx_common.cuh"
@@ -51,7 +52,7 @@ namespace hx {
 namespace pg {
 
 constexpr int BM = 128;            // rows of A per tile (TMEM lanes)
-constexpr uint64_t WAIT_LIMIT = 2000000000ull;
+constexpr uint64_t WAIT_LIMIT = 2000000000ull;  // ns
 constexpr int NAN_EXP = -(1 << 28);  // exponent of a row that holds an infinity or a NaN
 
 // Planes (NP), levels (LV), real columns per tile (BN), K' per stage (BK), stages per partial sum (CT), pipeline stages
@@ -112,6 +113,8 @@ struct PlaneArgs {
     const Cx* src;          // indexed like out
     typename Shape<T>::Acc* parts;  // scratch of a K split: one tile's sums per CTA
     int* status;
+    uint64_t wait_limit;    // ns (WAIT_LIMIT)
+    int stall;              // test of the waits: the first CTA along K loads nothing, so that its waits run out
 };
 
 // Words of the shared-memory descriptor of a K-major operand whose rows are ROW_BYTES wide and swizzled over that
@@ -397,6 +400,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         ptx::mbar_init(bar_done, 1);
         *abort_flag = 0;
         ptx::fence_mbar_init();
+        ptx::fence_cluster();  // the flag, before the cluster barrier's first phase
         ptx::prefetch_tensormap(&g.tmap_a);
         ptx::prefetch_tensormap(&g.tmap_b);
     }
@@ -415,6 +419,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
+    if (KS > 1) ptx::cluster_arrive_relaxed();  // waited for before a CTA writes another's flag: that has started by then
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t smem_a = ptx::smem_addr(smem);
     auto give_up = [&] {
@@ -426,10 +431,11 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         if (lane == 0) {
             int last_use[S::ST];
             for (int s = 0; s < S::ST; ++s) last_use[s] = -1;
-            for (int i = 0; i < nkt; ++i) {
+            const int loads = g.stall && ks == 0 ? 0 : nkt;
+            for (int i = 0; i < loads; ++i) {
                 if (*abort_flag) break;
                 const int s = i % S::ST, u = i / S::ST;
-                if (u > 0 && !ptx::mbar_wait_bounded(bar_empty(s), (u - 1) & 1, WAIT_LIMIT)) {
+                if (u > 0 && !ptx::mbar_wait_bounded(bar_empty(s), (u - 1) & 1, g.wait_limit)) {
                     give_up();
                     break;
                 }
@@ -442,7 +448,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
             }
             // No copy may land in shared memory after this CTA leaves the pipeline.
             for (int s = 0; s < S::ST; ++s)
-                if (last_use[s] >= 0 && !ptx::mbar_wait_bounded(bar_full(s), last_use[s] & 1, WAIT_LIMIT)) give_up();
+                if (last_use[s] >= 0 && !ptx::mbar_wait_bounded(bar_full(s), last_use[s] & 1, g.wait_limit)) give_up();
         }
     } else if (warp == 1) {
         // the whole warp runs this branch (see ptx::elect_one)
@@ -452,7 +458,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
             const int s = i % S::ST, u = i / S::ST;
             const int part = i / S::CT;
             const bool first = i % S::CT == 0, last = i % S::CT == S::CT - 1 || i == nkt - 1;
-            ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, WAIT_LIMIT));
+            ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, g.wait_limit));
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t a0 = desc_lo(smem_a + s * LY::STAGE);
@@ -460,7 +466,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
             constexpr uint32_t hi = desc_hi<LY::ROW_BYTES>();
             auto drained = [&](int l) {  // the accumulator's previous partial sum must have been read
                 if (ok)
-                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(l), (part - 1) & 1, WAIT_LIMIT));
+                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(l), (part - 1) & 1, g.wait_limit));
                 ptx::tc_fence_after();
             };
             // planes pb .. pb + count - 1 of B, which follow one another as the levels do in TMEM
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         }
         // TMEM and the pipeline buffers are released only after every MMA issued above
         if (leader) ptx::umma_commit(bar_done);
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_done, 0, WAIT_LIMIT)) && ok;
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_done, 0, g.wait_limit)) && ok;
         if (!ok && leader) give_up();
     }
     // ---- warps 2 and up: two or four per TMEM lane quarter, each a slice of the columns ---------------------------------
@@ -528,7 +534,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         for (int p = 0; p < nparts; ++p) {
             auto level = [&](auto lc) {
                 constexpr int l = decltype(lc)::value;
-                if (live && !ptx::mbar_wait_bounded(bar_ready(l), p & 1, WAIT_LIMIT)) give_up();
+                if (live && !ptx::mbar_wait_bounded(bar_ready(l), p & 1, g.wait_limit)) give_up();
                 // warp-uniform: the TMEM loads are .sync.aligned
                 live = __shfl_sync(0xffffffffu, (int)(live && *abort_flag == 0), 0) != 0;
                 if (!live) return;
@@ -564,16 +570,21 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     }
     if (KS > 1) {
         __syncwarp();
+        ptx::cluster_wait();
+        if (epi && et < KS && *abort_flag) {  // what this CTA lacks is missing from every slice of the columns
+            ptx::fence_cluster();
+            ptx::st_cluster_u32(ptx::map_shared_rank(ptx::smem_addr(const_cast<int*>(abort_flag)), et), 1);
+        }
+        __syncwarp();
         ptx::cluster_sync();  // every CTA's partial sums are written (release and acquire cover L2 too)
     }
     if (epi) {
         if (KS == 1) ptx::named_barrier(1, S::EPI);
-        if (*abort_flag == 0) {
-            if (KS == 1) finish_columns<T, 1>(g, part_s, others, s_cs, rs, m0, n_tile, 0, et);
-            else if (KS == 2) finish_columns<T, 2>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
-            else if (KS == 4) finish_columns<T, 4>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
-            else finish_columns<T, 8>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
-        }
+        if (*abort_flag) rs = NAN_EXP;  // sums that are not complete: every result of theirs is NaN
+        if (KS == 1) finish_columns<T, 1>(g, part_s, others, s_cs, rs, m0, n_tile, 0, et);
+        else if (KS == 2) finish_columns<T, 2>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+        else if (KS == 4) finish_columns<T, 4>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+        else finish_columns<T, 8>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
     }
     ptx::tc_fence_before();
     __syncthreads();

@@ -411,6 +411,8 @@ template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const 
     g.row_scale = (const typename Shape<T>::Scale*)a.scale;
     g.col_scale = (const typename Shape<T>::Scale*)b.scale;
     g.ktiles = a.kpitch / Shape<T>::BK;
+    g.stall = fault_injected("wait");
+    g.wait_limit = g.stall ? 10000000ull : WAIT_LIMIT;
     g.n_tiles = (int)ceil_div(b.n, LY::TN);
     const unsigned m_tiles = ceil_div(a.rows, BM);
     g.ksplit = k_split<T>((long long)m_tiles * g.n_tiles, g.ktiles, throughput);

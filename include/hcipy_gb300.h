@@ -190,8 +190,9 @@ HX_API int hx_intensity_sums_grad(const void* field, int dtype, long long n, int
                                   const double* grad, void* out, void* stream);
 
 /* Status of the plan's bounded device-side waits since the last reset: HX_OK, or
- * HX_ERR_TIMEOUT when a wait of the tensor-core GEMM gave up (its CTA then
- * returned without writing).  Synchronizes with the device; reset != 0 clears it. */
+ * HX_ERR_TIMEOUT when a wait of the tensor-core GEMM gave up (its part of the result
+ * is then NaN in FP32 and FP64 plans, and not written in split plans).  Synchronizes
+ * with the device; reset != 0 clears it. */
 HX_API int hx_mft_plan_status(const hx_mft_plan* plan, int reset);
 
 /* Tile policy of the plan's GEMMs, HX_SCHEDULE_LATENCY (default) or HX_SCHEDULE_THROUGHPUT, for plans whose
