@@ -20,7 +20,8 @@ void count_launch(int n = 1);
 
 // Host-side fault injection: when HX_FAULT names `site` ("alloc", "plan" or
 // "launch"), the entry point returns HX_ERR_INJECTED before touching the GPU.  "wait": the plain tensor-core GEMM runs with
-// a short limit on its waits and with a load left out, so that one of them runs out.
+// a short limit on its waits and with a load left out, so that one of them runs out.  "operand_memory" and "operand_map":
+// its operands find no memory, or no tensor map.
 bool fault_injected(const char* site);
 
 // Kernel timing (hx_trace_enable): a scope records a CUDA event on `stream` when it opens and another when it

@@ -486,9 +486,9 @@ int hx_mft_plan_create(int nx, int ny, int nu, int nv, const double* x, const do
             if ((rc = gen_matrix(dtype, ny, nv, dy, dv, +1.0, dwy, nullptr, &p->m1a, stream))) break;
             if ((rc = gen_matrix(dtype, nu, nx, du, dx, +1.0, nullptr, dwx, &p->m2a, stream))) break;
         }
-        if (hx::plane_mft_fits(nx, ny, nu, nv, dtype) &&
-            hx::plane_mft_create(dtype, nx, ny, nu, nv, dx, dy, du, dv, dwx, dwy, dwu, dwv, stream, &p->plane) != HX_OK)
-            cudaGetLastError();  // no memory for the cut operands: the plan runs on the CUDA cores
+        if (hx::plane_mft_fits(nx, ny, nu, nv, dtype, weighted_in || weighted_out) &&
+            (rc = hx::plane_mft_create(dtype, nx, ny, nu, nv, dx, dy, du, dv, dwx, dwy, dwu, dwv, stream, &p->plane)))
+            break;
     } while (false);
     cleanup();
     if (rc != HX_OK) {

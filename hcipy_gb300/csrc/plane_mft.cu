@@ -504,6 +504,7 @@ template <typename T> bool takes(const Dims& d, int batch) {
 template <typename T> int make_const(PlaneMat& m, int N, const double* a, const double* b, double sign,
                                      const double* wn, cudaStream_t st) {
     m.n = N;
+    if (fault_injected("operand_map")) return HX_ERR_INJECTED;
     HX_TRY(encode_map<T>(&m.map, m, Shape<T>::BN));
     plane_const_kernel<T><<<(unsigned)N, 256, 0, st>>>(m.K, m.Kp, a, b, sign, wn, m.planes, m.plane_stride(),
                                                        m.kpitch, (typename Shape<T>::Scale*)m.scale);
@@ -529,7 +530,12 @@ int create_t(PlaneMft* p, const double* x, const double* y, const double* u, con
     };
     Carver count(nullptr);
     layout(count);
-    HX_TRY(cuda_status(cudaMalloc(&p->mem, count.off), "cudaMalloc(plane MFT plan)"));
+    const cudaError_t mem = fault_injected("operand_memory") ? cudaErrorMemoryAllocation : cudaMalloc(&p->mem, count.off);
+    if (mem == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return HX_ERR_ALLOC;
+    }
+    HX_TRY(cuda_status(mem, "cudaMalloc(plane MFT plan)"));
     HX_TRY(cuda_status(cudaMemsetAsync(p->mem, 0, count.off, st), "memset plane MFT plan"));
     Carver c(p->mem);
     layout(c);
@@ -600,20 +606,20 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
 
 }  // namespace
 
-bool plane_mft_fits(int nx, int ny, int nu, int nv, int dtype) {
+bool plane_mft_fits(int nx, int ny, int nu, int nv, int dtype, bool weighted) {
     if (std::max(std::max(nx, ny), std::max(nu, nv)) > 8192) return false;
     if (std::min(std::min(nx, ny), std::min(nu, nv)) < 16) return false;
-    // operands of the two directions: at most 4 GB
-    const double bytes = 8.0 * (dtype == HX_C64 ? Shape<float>::NP : Shape<double>::NP) * 2.0 *
+    // The operands of the two directions, and of the adjoint where weights make it a third: at most 8 GB, 3% of the memory
+    // (complex64 transforms between uniform grids of 8192^2 points take 6.4).
+    const double bytes = 8.0 * (dtype == HX_C64 ? Shape<float>::NP : Shape<double>::NP) * (weighted ? 3.0 : 2.0) *
                          ((double)nx * nu + (double)ny * nv);
-    return bytes <= 4e9;
+    return bytes <= 8e9;
 }
 
 int plane_mft_create(int dtype, int nx, int ny, int nu, int nv, const double* x, const double* y, const double* u,
                      const double* v, const double* wx, const double* wy, const double* wu, const double* wv,
                      cudaStream_t st, PlaneMft** out) {
     *out = nullptr;
-    if (!get_encode()) return HX_ERR_UNSUPPORTED;
     PlaneMft* p = new PlaneMft();
     p->dtype = dtype;
     p->nx = nx, p->ny = ny, p->nu = nu, p->nv = nv;
@@ -621,7 +627,7 @@ int plane_mft_create(int dtype, int nx, int ny, int nu, int nv, const double* x,
                                    : create_t<double>(p, x, y, u, v, wx, wy, wu, wv, st);
     if (rc != HX_OK) {
         plane_mft_destroy(p);
-        return rc;
+        return rc == HX_ERR_ALLOC ? (int)HX_OK : rc;  // no room for the cut operands: the plan runs on the CUDA cores
     }
     *out = p;
     return HX_OK;
