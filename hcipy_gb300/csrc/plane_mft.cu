@@ -465,7 +465,7 @@ template <typename T> struct Pass {
 };
 
 template <typename T> size_t carve_pass(void* ws, const Dims& d, int fields, Pass<T>* out) {
-    Carver c(ws);
+    Carver c((void*)(((uintptr_t)ws + 255) / 256 * 256));  // TMA wants 16 bytes; a caller's scratch may start anywhere
     Pass<T> q;
     const long long r1 = (long long)fields * d.K1, r2 = (long long)fields * d.C;
     carve_mat<T>(c, q.s1, r1, r1, d.K2);
@@ -477,7 +477,7 @@ template <typename T> size_t carve_pass(void* ws, const Dims& d, int fields, Pas
         return ks > 1 ? (size_t)tiles * ks * Layout<T>::TN * 2 * BM * sizeof(typename Shape<T>::Acc) : (size_t)0;
     };
     q.parts = c.take(std::max(part_bytes(q.s1, d.C), part_bytes(q.s2, d.R)));
-    q.bytes = c.off + 256;
+    q.bytes = c.off + 255;
     q.fields = fields;
     if (out) *out = q;
     return q.bytes;
