@@ -71,7 +71,7 @@ def _quintic_taps(shift):
     for offset in (2.0 + f, 1.0 + f, f, 1.0 - f, 2.0 - f, 3.0 - f):
         acc, x = 0.0, offset + 3.0
         for c in _QUINTIC:
-            if x <= 0.0:  # x only falls: the terms that follow are zero
+            if not x > 0.0:  # x only falls: the terms that follow are zero (not-a-number has none)
                 break
             acc += c * x**5
             x -= 1.0
