@@ -518,8 +518,16 @@ bool y_first(const hx_fft_plan* p, int direction) {
            n_src[1] * (double)p->N[0] + column * n_dst[0] * (double)p->N[1];
 }
 
+// Bytes of the intermediate between the two passes of a 2-D transform.
+size_t mid_bytes(const hx_fft_plan* p, int direction, int batch, bool y) {
+    const bool fwd = direction == HX_FORWARD;
+    const int* n_src = fwd ? p->n_in : p->n_out;
+    const int* n_dst = fwd ? p->n_out : p->n_in;
+    return p->esize * (size_t)batch * (y ? (size_t)n_dst[1] * n_src[0] : (size_t)n_src[1] * n_dst[0]);
+}
+
 template <typename T>
-int fft_execute_t(const hx_fft_plan* p, int direction, int batch, const void* in, void* out, void* ws,
+int fft_execute_t(const hx_fft_plan* p, int direction, int batch, const void* in, void* out, void* ws, bool y,
                   cudaStream_t s) {
     const bool fwd = direction == HX_FORWARD;
     const int sign = fwd ? -1 : 1;
@@ -546,7 +554,7 @@ int fft_execute_t(const hx_fft_plan* p, int direction, int batch, const void* in
     }
     const long long src_sz = (long long)n_src[0] * n_src[1];
     const long long dst_sz = (long long)n_dst[0] * n_dst[1];
-    if (y_first(p, direction)) {
+    if (y) {
         // pass y: columns of the source (n_src[0] lines, stride n_src[0]) -> intermediate (n_dst[1] x n_src[0])
         const long long mid_sz = (long long)n_dst[1] * n_src[0];
         HX_TRY(fft_pass<T>(p, 1, sign, batch, n_src[0], in, 1, n_src[0], src_sz, n_src[1], c_src[1], src_fac(1), ws, 1,
@@ -610,11 +618,7 @@ int hx_fft_plan_create(int ndim, const int* in_dims, const int* internal_dims, c
 
 size_t hx_fft_workspace_bytes(const hx_fft_plan* p, int direction, int batch) {
     if (!p || p->ndim == 1 || batch <= 0) return 0;
-    const bool fwd = direction == HX_FORWARD;
-    const int* n_src = fwd ? p->n_in : p->n_out;
-    const int* n_dst = fwd ? p->n_out : p->n_in;
-    return p->esize * (size_t)batch *
-           (y_first(p, direction) ? (size_t)n_dst[1] * n_src[0] : (size_t)n_src[1] * n_dst[0]);
+    return mid_bytes(p, direction, batch, y_first(p, direction));
 }
 
 int hx_fft_execute(const hx_fft_plan* p, int direction, int batch, const void* in, void* out, void* ws,
@@ -623,13 +627,16 @@ int hx_fft_execute(const hx_fft_plan* p, int direction, int batch, const void* i
     HX_CHECK_ARG(direction == HX_FORWARD || direction == HX_BACKWARD, "hx_fft_execute: unknown direction %d",
                  direction);
     HX_CHECK_ARG(batch >= 1 && in && out, "hx_fft_execute: bad batch or NULL field");
-    const size_t need = hx_fft_workspace_bytes(p, direction, batch);
+    // Scratch for the rows-first order alone is enough too: between rectangular grids it can be the smaller one.
+    bool y = p->ndim == 2 && y_first(p, direction);
+    if (y && ws_bytes < mid_bytes(p, direction, batch, true)) y = false;
+    const size_t need = p->ndim == 1 ? 0 : mid_bytes(p, direction, batch, y);
     HX_CHECK_ARG(ws_bytes >= need && (need == 0 || ws != nullptr), "hx_fft_execute: workspace of %zu bytes needed",
                  need);
     if (hx::fault_injected("launch")) return HX_ERR_INJECTED;
     cudaStream_t s = (cudaStream_t)stream;
-    if (p->dtype == HX_C64) return fft_execute_t<float>(p, direction, batch, in, out, ws, s);
-    return fft_execute_t<double>(p, direction, batch, in, out, ws, s);
+    if (p->dtype == HX_C64) return fft_execute_t<float>(p, direction, batch, in, out, ws, y, s);
+    return fft_execute_t<double>(p, direction, batch, in, out, ws, y, s);
 }
 
 int hx_fft_plan_destroy(hx_fft_plan* p) {

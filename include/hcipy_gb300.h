@@ -252,7 +252,9 @@ HX_API int hx_fft_plan_create(int ndim, const int* in_dims, const int* internal_
                        const double* const* pre, const double* const* post,
                        double scale_re, double scale_im, int dtype, void* stream, hx_fft_plan** plan);
 HX_API size_t hx_fft_workspace_bytes(const hx_fft_plan* plan, int direction, int batch);
-/* direction HX_FORWARD (input plane -> output plane) or HX_BACKWARD. */
+/* direction HX_FORWARD (input plane -> output plane) or HX_BACKWARD.  The transform takes the order of its axes for
+ * which hx_fft_workspace_bytes asks, or, given scratch for that only, rows first (batch x source rows x destination
+ * columns elements). */
 HX_API int hx_fft_execute(const hx_fft_plan* plan, int direction, int batch, const void* in, void* out,
                    void* workspace, size_t workspace_bytes, void* stream);
 HX_API int hx_fft_plan_destroy(hx_fft_plan* plan);
