@@ -510,9 +510,12 @@ int fft_pass(const hx_fft_plan* p, int d, int sign, int batch, int nlines,
 }
 
 // Which axis of a 2-D transform goes first.  The two orders run n_src[1] rows and n_dst[0] columns, or n_src[0] columns
-// and n_dst[1] rows; a column pass is the slower one (strided lines, of which a CTA holds two to four, in segments of 16
-// to 32 bytes: 129 us for 4096 columns of 4096 points against 28 us for 1024 rows), so a zero-padded transform takes
-// its few columns first and a cropped one last.
+// and n_dst[1] rows.  A column pass is the slower one in complex64 (strided lines, in segments of 16 to 32 bytes), so a
+// zero-padded transform takes its few columns first and a cropped one last.  Both orders of square complex64 fields, rows
+// or columns first: 1024^2 to 4096^2 100 and 89 us, back 101 and 121; 437^2 to 874^2 61 and 55, back 55 and 60; 640^2 to
+// 1920^2 146 and 139, back 140 and 141; at worst 333^2 to 999^2 113 and 117.  With 1.3 the rule takes the better one within
+// 5% over 22 such grids, between rectangular ones within 20% (1000 x 250 to 2000 x 500: 43 and 51).  In complex128, bound
+// by the float64 pipe, either order is within 1.5% of the other.
 bool y_first(const hx_fft_plan* p, int direction) {
     const bool fwd = direction == HX_FORWARD;
     const int* n_src = fwd ? p->n_in : p->n_out;
