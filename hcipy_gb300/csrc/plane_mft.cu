@@ -568,8 +568,12 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
     using Cx = typename cplx<T>::type;
     const Dims d = dims_of(p, direction);
     const int per = fields_per_pass<T>(d, batch);
-    for (int b0 = 0; b0 < batch; b0 += per) {
-        const int nb = std::min(per, batch - b0);
+    // Fields that grow are taken from the last on: a result written over its own input (out == in) then lies past the inputs
+    // of the passes still to come; fields that shrink lie before them.
+    const bool grow = (long long)d.R * d.C > (long long)d.K1 * d.K2;
+    const int passes = (batch + per - 1) / per;
+    for (int i = 0; i < passes; ++i) {
+        const int b0 = (grow ? passes - 1 - i : i) * per, nb = std::min(per, batch - b0);
         Pass<T> q;
         carve_pass<T>(ws, d, nb, &q);
         const Cx* src_f = (const Cx*)in + (long long)b0 * d.K1 * d.K2;
