@@ -5,40 +5,46 @@
 // warp (consecutive m) store consecutive addresses straight from the accumulators, and so that the second GEMM of a
 // transform reads the first one's result by contiguous rows.
 //
-// Operands.  Every row of A and of B is scaled by a power of two and cut into fp16 planes of balanced digits,
-// x = 2^E sum_i d_i w_i with |x| <= 2^E:
-//   complex64 : three digits of base 512, d_i in [-256, 256], w_i = 2^(-8 - 9 i), which leaves 2^-27 of 2^E at most;
+// Operands.  Every row of A and of B is scaled by a power of two and cut into fp16 planes, in one of three forms (plane_mft.cu
+// says which a complex64 operand takes):
+//   C64Digits : x = 2^E sum_i d_i 2^(-8 - 9 i) with |x| <= 2^E, three digits of base 512, d_i in [-256, 256], to 2^-27 of 2^E;
 //               the six products d_i d_j with i + j <= 2 go to three accumulators, one per level i + j;
-//   complex128: seven digits of base 256, d_i in [-128, 128], w_i = 2^(-7 - 8 i), which leaves 2^-56; the 28 products
-//               with i + j <= 6 go to seven accumulators.
+//   C64Floats : x = s (h + l), h and l the fp16 roundings of x / s and of x / s - h, which keeps 22 bits of every element;
+//               the products h l, l h and h h go to one FP32 accumulator, the small ones first;
+//   C128Digits: x = 2^E sum_i d_i 2^(-7 - 8 i), seven digits of base 256, d_i in [-128, 128], to 2^-56 of 2^E; the 28
+//               products with i + j <= 6 go to seven accumulators.
 // A holds [Ar | Ai] per row (K' = 2K), B holds the complex embedding in blocks of 8 complex columns: the 8 real
 // columns [Br | -Bi], then the 8 imaginary ones [Bi | Br].
 //
 // Sums.  The tensor cores truncate an FP32 sum that no longer fits 24 bits (a sum of 4096 positive products comes out
-// 2.5e-5 low, of 64 products 1.5e-7 low: measured against float64), so the accumulators hold whole numbers that fit:
-//   complex64 : 256 terms of K': level 0 is at most 256 * 2^16 = 2^24, hence exact, and is added to 32-bit integers (2^30
+// 2.5e-5 low, of 64 products 1.5e-7 low: measured against float64), so no accumulator runs long:
+//   C64Digits : 256 terms of K': level 0 is at most 256 * 2^16 = 2^24, hence exact, and is added to 32-bit integers (2^30
 //               over the longest K' of 16384).  Levels 1 and 2 weigh 2^-9 and 2^-18 of it: what they lose below 24 bits is
-//               below 2^-32 of the terms' size.  They are added in FP32, and the sum is rounded once, at the end.
-//   complex128: 128 terms: every level is below 7 * 128 * 2^14 < 2^24, hence exact, and is added to 64-bit integers
+//               below 2^-32 of the terms' size.  They are added in FP32, and the sum is rounded once, at the end;
+//   C64Floats : 32 terms of K', then the accumulator is added to FP32 registers in round-to-nearest, in blocks of 16
+//               partial sums.  Such a sum is truncated after its first 16 terms and at the end, by half an ulp on
+//               average: 2^-24 / (2 ln 2) = 4.3e-8 of a value with mantissas spread over their logarithm, and half of
+//               that for the first truncation, 6.4e-8 together (6.5e-8 measured).  A factor so close to 1 on every
+//               GEMM adds up along a chain of transforms, so it is taken back on average (Sums<C64Floats>::add);
+//   C128Digits: 128 terms: every level is below 7 * 128 * 2^14 < 2^24, hence exact, and is added to 64-bit integers
 //               (levels 0-3 in one, 4-6 in another), exact over any K the plans take.
-// The error of a transform is that of its operands (above), of the dropped products (digits 1 and 2 in complex64: 2^-26 of the
-// two scales at most) and one rounding of each sum: 3.5-7.5e-8 for complex64, 1e-7 for gradients through six transforms.
-// Two planes of floating fp16 values with three products, 22 bits and FP32 sums of 32 terms were a quarter faster (Lyot
-// pass below 333 us), but what the truncated sums lost (6e-8 of their value on average) added up along a chain: such
-// gradients came out 3.6-5.3e-7 off where the CUDA cores give 2.6-3.5e-7, and a field of one pixel 1.0-2.2e-7 where they
-// give 0.4-0.6e-7.
+// The error of a transform in digits is that of its operands (above), of the dropped products (of digits 1 and 2 in complex64:
+// 2^-26 of the two scales at most) and one rounding of each sum: 3.5-7.5e-8 in complex64.  In floating planes it is
+// 1.1-2.0e-7, where the CUDA cores' sums of as many terms are 5e-7 to 1.6e-6 off.
 //
 // Pipeline.  One CTA per 128 rows x BN real columns (BN = 128 for complex64, 64 for complex128, whose seven levels
 // take 448 of the 512 TMEM columns): warp 0 issues TMA boxes of all planes of a K step, warp 1 the MMAs, the others
-// drain.  Each level has its own pair of barriers, so level l of the next partial sum starts as soon as level l of this
-// one is drained, in the order in which the next step's MMAs reach them.
+// drain.  Each accumulator has its own pair of barriers, so level l of the next partial sum starts as soon as level l of
+// this one is drained, in the order in which the next step's MMAs reach them; floating planes have four sets of their one
+// accumulator, two partial sums of a stage in each half.
 // With few tiles the CTAs of a thread-block cluster split K and add their partial sums in rank order, each CTA
 // finishing a slice of the columns.  The sums travel through L2 under the cluster's barrier: through distributed shared
 // memory they moved at 7 to 13 bytes per clock and SM.
-// Measured against the GEMMs on the CUDA cores: a complex128 lens of 512^2 points to 256^2 1060 -> 72 us (float64 pipe), a
-// complex64 Lyot pass over four fields of 1024^2 points 1700 -> 431 us (FP32 pipe).  complex64 is bound by shared memory (per
-// 16 K' its MMAs read 40 KB in 384 clocks while the loads write 24 KB, and it moves 128 bytes a clock), complex128 by the
-// epilogue (10 of 38 thousand clocks are MMAs where K is split eight ways).
+// Measured against the GEMMs on the CUDA cores: a complex128 lens of 512^2 points to 256^2 1060 -> 73 us (float64 pipe), a
+// complex64 Lyot pass over four fields of 1024^2 points 1700 -> 333 us in floating planes, 434 us in digits (FP32 pipe).
+// complex64 is bound by shared memory, which moves 128 bytes a clock: per 16 K' the MMAs of digits read 40 KB in 384 clocks
+// while the loads write 24 KB, those of floating planes 24 and 16 KB in 192 (1270 clocks per 64 K' measured).  complex128
+// is bound by the epilogue (10 of 38 thousand clocks are MMAs where K is split eight ways).
 // All waits are bounded (2 s): a wait that runs out records HX_ERR_TIMEOUT in the plan's status word, and the CTA, with the
 // others of its cluster, writes NaN instead of sums that are not complete, so that no result looks like one.
 #pragma once
@@ -55,27 +61,44 @@ constexpr int BM = 128;            // rows of A per tile (TMEM lanes)
 constexpr uint64_t WAIT_LIMIT = 2000000000ull;  // ns
 constexpr int NAN_EXP = -(1 << 28);  // exponent of a row that holds an infinity or a NaN
 
-// Planes (NP), levels (LV), real columns per tile (BN), K' per stage (BK), stages per partial sum (CT), pipeline stages
-// (ST), epilogue threads (EPI: the conversions at the end want warps).
-template <typename T> struct Shape;
-template <> struct Shape<float> {
-    static constexpr int NP = 3, LV = 3, BN = 128, BK = 32, CT = 8, ST = 4, EPI = 512;
+// The three forms of an operand.
+struct C64Digits {};   // complex64, three digits
+struct C64Floats {};   // complex64, two floating planes
+struct C128Digits {};  // complex128, seven digits
+
+// Element type (T), planes (NP), levels (LV), real columns per tile (BN), K' per stage (BK), accumulator sets (SETS), stages
+// per partial sum (CT) and partial sums per stage (PPS), pipeline stages (ST), epilogue threads (EPI: floating planes drain
+// often and little, digits seldom and much, and their conversions want warps).
+template <typename F> struct Shape;
+template <> struct Shape<C64Digits> {
+    using T = float;
+    static constexpr int NP = 3, LV = 3, BN = 128, BK = 32, SETS = 1, CT = 8, PPS = 1, ST = 4, EPI = 512;
     struct __align__(8) Acc {
         int hi;    // value = hi 2^-16 + lo 2^-34 (times the scales)
         float lo;
     };
     using Scale = int;  // exponent of the power-of-two scale
+    static __device__ Scale poison() { return NAN_EXP; }
 };
-template <> struct Shape<double> {
-    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, CT = 4, ST = 2, EPI = 512;
+template <> struct Shape<C64Floats> {
+    using T = float;
+    static constexpr int NP = 2, LV = 1, BN = 128, BK = 64, SETS = 4, CT = 1, PPS = 2, ST = 3, EPI = 256;
+    using Acc = float;
+    using Scale = float;
+    static __device__ Scale poison() { return __int_as_float(0x7fc00000); }
+};
+template <> struct Shape<C128Digits> {
+    using T = double;
+    static constexpr int NP = 7, LV = 7, BN = 64, BK = 32, SETS = 1, CT = 4, PPS = 1, ST = 2, EPI = 512;
     struct __align__(16) Acc {
         long long hi, lo;  // value = hi 2^-38 + lo 2^-62 (times the scales)
     };
-    using Scale = int;  // exponent of the power-of-two scale
+    using Scale = int;
+    static __device__ Scale poison() { return NAN_EXP; }
 };
 
-template <typename T> struct Layout {
-    using S = Shape<T>;
+template <typename F> struct Layout {
+    using S = Shape<F>;
     static constexpr int ROW_BYTES = S::BK * 2;  // 128 (128-byte swizzle) or 64 (64-byte swizzle)
     static constexpr int A_PLANE = BM * ROW_BYTES;
     static constexpr int B_PLANE = S::BN * ROW_BYTES;
@@ -86,23 +109,24 @@ template <typename T> struct Layout {
     static constexpr int THREADS = S::EPI + 64;     // TMA warp, MMA warp, epilogue warps
     static constexpr int COLS = S::BN / (S::EPI / BM);  // real columns per epilogue thread
     static constexpr int LD = COLS < 32 ? COLS : 32;    // columns per TMEM load
+    static constexpr int NACC = S::SETS * S::LV;
     static constexpr int TMEM_COLS = 512;
-    static_assert(S::LV * S::BN <= TMEM_COLS, "the accumulators must fit TMEM");
+    static_assert(NACC * S::BN <= TMEM_COLS, "the accumulators must fit TMEM");
     static_assert(BM * S::BN * (int)sizeof(typename S::Acc) <= PIPE, "partial sums must fit the pipeline buffers");
     static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
 };
 
-template <typename T>
+template <typename F>
 struct PlaneArgs {
-    using Cx = typename cplx<T>::type;
+    using Cx = typename cplx<typename Shape<F>::T>::type;
     CUtensorMap tmap_a;
     CUtensorMap tmap_b;
     int ktiles;             // K' / BK
     int ksplit;             // CTAs along K per tile (the size of the cluster)
     int n_tiles;
     int M, N;               // rows of A, complex columns
-    const typename Shape<T>::Scale* row_scale;
-    const typename Shape<T>::Scale* col_scale;
+    const typename Shape<F>::Scale* row_scale;
+    const typename Shape<F>::Scale* col_scale;
     int rows_per_field;     // row m is row m % rows_per_field of field m / rows_per_field
     long long ldo, out_z;   // element (m, n): out[field * out_z + n * ldo + row of the field]
     Cx* out;
@@ -111,7 +135,7 @@ struct PlaneArgs {
     int epi;                // HX_EPI_*
     const Cx* mask;         // one field, indexed n * ldo + row
     const Cx* src;          // indexed like out
-    typename Shape<T>::Acc* parts;  // scratch of a K split: one tile's sums per CTA
+    typename Shape<F>::Acc* parts;  // scratch of a K split: one tile's sums per CTA
     int* status;
     uint64_t wait_limit;    // ns (WAIT_LIMIT)
     int stall;              // test of the waits: the first CTA along K loads nothing, so that its waits run out
@@ -178,68 +202,105 @@ __device__ __forceinline__ float fixed_to_float(int hi, float lo, int e) {
     return v * __int_as_float((h + 127) << 23) * __int_as_float((c - h + 127) << 23);
 }
 
-__device__ __forceinline__ float acc_value(const Shape<float>::Acc& a, int re, int ce, bool& rare) {
+__device__ __forceinline__ float acc_value(const Shape<C64Digits>::Acc& a, int re, int ce, bool& rare) {
     rare |= re == NAN_EXP || ce == NAN_EXP;
     return fixed_to_float(a.hi, a.lo, re + ce - 34);
 }
-__device__ __forceinline__ double acc_value(const Shape<double>::Acc& a, int re, int ce, bool& rare) {
+__device__ __forceinline__ double acc_value(const Shape<C128Digits>::Acc& a, int re, int ce, bool& rare) {
     rare |= re == NAN_EXP || ce == NAN_EXP;
     return fixed_to_double(a.hi, a.lo, re + ce - 62, rare);
 }
-__device__ __forceinline__ float acc_rare(const Shape<float>::Acc& a, int re, int ce) {
+__device__ __forceinline__ float acc_rare(const Shape<C64Digits>::Acc& a, int re, int ce) {
     if (re == NAN_EXP || ce == NAN_EXP) return __int_as_float(0x7fc00000);
     return fixed_to_float(a.hi, a.lo, re + ce - 34);
 }
-__device__ __forceinline__ double acc_rare(const Shape<double>::Acc& a, int re, int ce) {
+__device__ __forceinline__ double acc_rare(const Shape<C128Digits>::Acc& a, int re, int ce) {
     if (re == NAN_EXP || ce == NAN_EXP) return __longlong_as_double(0x7ff8000000000000ll);
     return scaled_value(a.hi, a.lo, re + ce - 62);
 }
 
+__device__ __forceinline__ float acc_value(const float& a, float rs, float cs, bool&) { return a * cs * rs; }
+__device__ __forceinline__ float acc_rare(const float& a, float rs, float cs) { return a * cs * rs; }
+
+__device__ __forceinline__ void acc_add(float& a, const float& b) { a += b; }
 template <typename A> __device__ __forceinline__ void acc_add(A& a, const A& b) {
     a.hi += b.hi;
     a.lo += b.lo;
 }
 
 // Partial sums of the other CTAs of a K split travel through L2.
-__device__ __forceinline__ void put_part(Shape<float>::Acc* p, const Shape<float>::Acc& v) {
+__device__ __forceinline__ void put_part(float* p, float v) { __stcg(p, v); }
+__device__ __forceinline__ float get_part(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ void put_part(Shape<C64Digits>::Acc* p, const Shape<C64Digits>::Acc& v) {
     __stcg(reinterpret_cast<int2*>(p), make_int2(v.hi, __float_as_int(v.lo)));
 }
-__device__ __forceinline__ void put_part(Shape<double>::Acc* p, const Shape<double>::Acc& v) {
+__device__ __forceinline__ void put_part(Shape<C128Digits>::Acc* p, const Shape<C128Digits>::Acc& v) {
     __stcg(reinterpret_cast<longlong2*>(p), make_longlong2(v.hi, v.lo));
 }
-__device__ __forceinline__ Shape<float>::Acc get_part(const Shape<float>::Acc* p) {
+__device__ __forceinline__ Shape<C64Digits>::Acc get_part(const Shape<C64Digits>::Acc* p) {
     const int2 v = __ldcg(reinterpret_cast<const int2*>(p));
     return {v.x, __int_as_float(v.y)};
 }
-__device__ __forceinline__ Shape<double>::Acc get_part(const Shape<double>::Acc* p) {
+__device__ __forceinline__ Shape<C128Digits>::Acc get_part(const Shape<C128Digits>::Acc* p) {
     const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(p));
     return {v.x, v.y};
 }
 
 // Running sums of one thread's columns.
-template <typename T> struct Sums;
-template <> struct Sums<float> {
-    static constexpr int COLS = Layout<float>::COLS;
-    Shape<float>::Acc a[COLS];
-    __device__ __forceinline__ void clear() {
+template <typename F> struct Sums;
+template <> struct Sums<C64Digits> {
+    static constexpr int COLS = Layout<C64Digits>::COLS;
+    Shape<C64Digits>::Acc a[COLS];
+    __device__ __forceinline__ void start(int, int) {
 #pragma unroll
         for (int j = 0; j < COLS; ++j) a[j] = {0, 0.0f};
     }
     // level 0 in units of its own, levels 1 and 2 (2^9 and 1) in units of level 2
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
 #pragma unroll
-        for (int j = 0; j < Layout<float>::LD; ++j) {
+        for (int j = 0; j < Layout<C64Digits>::LD; ++j) {
             if (L == 0) a[j0 + j].hi += __float2int_rn(v[j]);
             else if (L == 1) a[j0 + j].lo = fmaf(v[j], 512.0f, a[j0 + j].lo);
             else a[j0 + j].lo += v[j];
         }
     }
-    __device__ __forceinline__ const Shape<float>::Acc& get(int j) const { return a[j]; }
+    __device__ __forceinline__ void end_partial(bool) {}
+    __device__ __forceinline__ const Shape<C64Digits>::Acc& get(int j) const { return a[j]; }
 };
-template <> struct Sums<double> {
-    static constexpr int COLS = Layout<double>::COLS;
-    Shape<double>::Acc a[COLS];
-    __device__ __forceinline__ void clear() {
+template <> struct Sums<C64Floats> {
+    static constexpr int COLS = Layout<C64Floats>::COLS;
+    float tot[COLS], blk[COLS];
+    int n = 0, q, half;
+    __device__ __forceinline__ void start(int half_, int first) {
+        half = half_;
+        q = first % half_;
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) tot[j] = blk[j] = 0.0f;
+    }
+    // Every second partial sum times 1 + 2^-23, in the one rounding of the addition: 6.0e-8 of the 6.4e-8 that truncated sums
+    // lose on average.  Counted from the start of either half of K', so that real and imaginary fields fare alike.  A sum
+    // of one or few terms (a field of few pixels) may have lost nothing; its transform is then up to 2^-23 too large per GEMM,
+    // 1.0-2.2e-7 in all where the CUDA cores are 0.4-0.6e-7 off.
+    template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
+        const float w = (q & 1) ? 1.0f : 1.0f + 0x1p-23f;
+#pragma unroll
+        for (int j = 0; j < Layout<C64Floats>::LD; ++j) blk[j0 + j] = fmaf(v[j], w, blk[j0 + j]);
+    }
+    __device__ __forceinline__ void end_partial(bool last) {
+        if (++q == half) q = 0;
+        if ((++n & 15) != 0 && !last) return;
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) {
+            tot[j] += blk[j];
+            blk[j] = 0.0f;
+        }
+    }
+    __device__ __forceinline__ float get(int j) const { return tot[j]; }
+};
+template <> struct Sums<C128Digits> {
+    static constexpr int COLS = Layout<C128Digits>::COLS;
+    Shape<C128Digits>::Acc a[COLS];
+    __device__ __forceinline__ void start(int, int) {
 #pragma unroll
         for (int j = 0; j < COLS; ++j) a[j] = {0, 0};
     }
@@ -247,13 +308,14 @@ template <> struct Sums<double> {
     template <int L> __device__ __forceinline__ void add(int j0, const float* v) {
         constexpr int W = L < 4 ? 1 << (8 * (3 - L)) : 1 << (8 * (6 - L));
 #pragma unroll
-        for (int j = 0; j < Layout<double>::LD; ++j) {
+        for (int j = 0; j < Layout<C128Digits>::LD; ++j) {
             const long long p = (long long)__float2int_rn(v[j]) * W;
             if (L < 4) a[j0 + j].hi += p;
             else a[j0 + j].lo += p;
         }
     }
-    __device__ __forceinline__ const Shape<double>::Acc& get(int j) const { return a[j]; }
+    __device__ __forceinline__ void end_partial(bool) {}
+    __device__ __forceinline__ const Shape<C128Digits>::Acc& get(int j) const { return a[j]; }
 };
 
 // f with the compile-time numbers 0 .. N - 1.
@@ -268,15 +330,16 @@ template <int N, typename F> __device__ __forceinline__ void each_level(F&& f) {
 // columns, the CTA's own partial sums from shared memory and the others' from `others` (L2), added in rank order.
 // Lanes along the rows, so that the reads and the stores are contiguous; U columns at a time, their loads ahead of
 // their arithmetic.
-template <typename T, int KS>
-__device__ __forceinline__ void finish_columns(const PlaneArgs<T>& g, const typename Shape<T>::Acc* part_s,
-                                               const typename Shape<T>::Acc* others,
-                                               const typename Shape<T>::Scale* s_cs, typename Shape<T>::Scale rs,
+template <typename F, int KS>
+__device__ __forceinline__ void finish_columns(const PlaneArgs<F>& g, const typename Shape<F>::Acc* part_s,
+                                               const typename Shape<F>::Acc* others,
+                                               const typename Shape<F>::Scale* s_cs, typename Shape<F>::Scale rs,
                                                int m0, int n_tile, int ks, int et) {
+    using T = typename Shape<F>::T;
     using Cx = typename cplx<T>::type;
-    using Acc = typename Shape<T>::Acc;
-    constexpr int TN = Layout<T>::TN, STEP = Shape<T>::EPI / BM, TNS = TN / KS;
-    constexpr int UMAX = sizeof(T) == 4 && KS < 4 ? 4 : 2, U = TNS / STEP < UMAX ? TNS / STEP : UMAX;
+    using Acc = typename Shape<F>::Acc;
+    constexpr int TN = Layout<F>::TN, STEP = Shape<F>::EPI / BM, TNS = TN / KS;
+    constexpr int UMAX = sizeof(Acc) == 4 || (sizeof(Acc) == 8 && KS < 4) ? 4 : 2, U = TNS / STEP < UMAX ? TNS / STEP : UMAX;
     static_assert(TNS % (STEP * U) == 0, "whole batches");
     constexpr int PART = TN * 2 * BM;  // one CTA's partial sums
     const int r = et & (BM - 1), m = m0 + r;
@@ -355,17 +418,16 @@ __device__ __forceinline__ void finish_columns(const PlaneArgs<T>& g, const type
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const __grid_constant__ PlaneArgs<T> g) {
-    using S = Shape<T>;
-    using LY = Layout<T>;
-    using Cx = typename cplx<T>::type;
+template <typename F>
+__global__ void __launch_bounds__(Layout<F>::THREADS, 1) plane_gemm_kernel(const __grid_constant__ PlaneArgs<F> g) {
+    using S = Shape<F>;
+    using LY = Layout<F>;
     using Acc = typename S::Acc;
     extern __shared__ __align__(1024) uint8_t pg_smem[];
     const uint32_t raw = ptx::smem_addr(pg_smem);
     uint8_t* smem = pg_smem + ((1024 - (raw & 1023)) & 1023);
     uint8_t* extra = smem + LY::PIPE;
-    // full[ST], empty[ST], ready[LV], drained[LV], done
+    // full[ST], empty[ST], ready[NACC], drained[NACC], done
     uint64_t* bars = reinterpret_cast<uint64_t*>(extra);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(extra + 256);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(extra + 260);
@@ -374,9 +436,9 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     auto bar_full = [&](int s) { return ptx::smem_addr(&bars[s]); };
     auto bar_empty = [&](int s) { return ptx::smem_addr(&bars[S::ST + s]); };
     auto bar_ready = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + a]); };
-    auto bar_drained = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + S::LV + a]); };
-    const uint32_t bar_done = ptx::smem_addr(&bars[2 * S::ST + 2 * S::LV]);
-    static_assert((2 * S::ST + 2 * S::LV + 1) * 8 <= 256, "barriers");
+    auto bar_drained = [&](int a) { return ptx::smem_addr(&bars[2 * S::ST + LY::NACC + a]); };
+    const uint32_t bar_done = ptx::smem_addr(&bars[2 * S::ST + 2 * LY::NACC]);
+    static_assert((2 * S::ST + 2 * LY::NACC + 1) * 8 <= 256, "barriers");
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform
     const int KS = g.ksplit;
@@ -393,7 +455,7 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
             ptx::mbar_init(bar_full(s), 1);
             ptx::mbar_init(bar_empty(s), 1);
         }
-        for (int a = 0; a < S::LV; ++a) {
+        for (int a = 0; a < LY::NACC; ++a) {
             ptx::mbar_init(bar_ready(a), 1);
             ptx::mbar_init(bar_drained(a), S::EPI / 32);
         }
@@ -456,56 +518,77 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
         bool ok = true;
         for (int i = 0; i < nkt && ok; ++i) {
             const int s = i % S::ST, u = i / S::ST;
-            const int part = i / S::CT;
+            const int part = i / S::CT * S::PPS, use = part / S::SETS;  // a stage's partial sums are of one use
+            const int set = part % S::SETS;
             const bool first = i % S::CT == 0, last = i % S::CT == S::CT - 1 || i == nkt - 1;
             ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_full(s), u & 1, g.wait_limit));
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t a0 = desc_lo(smem_a + s * LY::STAGE);
             const uint32_t b0 = a0 + (S::NP * LY::A_PLANE >> 4);
+            const uint32_t d0 = tmem + set * (S::LV * S::BN);
             constexpr uint32_t hi = desc_hi<LY::ROW_BYTES>();
             auto drained = [&](int l) {  // the accumulator's previous partial sum must have been read
                 if (ok)
-                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(l), (part - 1) & 1, g.wait_limit));
+                    ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(bar_drained(set * S::LV + l), (use - 1) & 1,
+                                                                        g.wait_limit));
                 ptx::tc_fence_after();
             };
             // planes pb .. pb + count - 1 of B, which follow one another as the levels do in TMEM
             auto mma = [&](auto count, int pa, int pb, int l, int kk, bool start) {
                 constexpr uint32_t idesc = ptx::umma_idesc_f16(BM, S::BN * decltype(count)::value);
                 if (leader)
-                    ptx::umma_f16_lo(tmem + l * S::BN, a0 + ((pa * LY::A_PLANE + kk * 32) >> 4),
+                    ptx::umma_f16_lo(d0 + l * S::BN, a0 + ((pa * LY::A_PLANE + kk * 32) >> 4),
                                      b0 + ((pb * LY::B_PLANE + kk * 32) >> 4), hi, idesc, start);
             };
             using one = std::integral_constant<int, 1>;
-            // The first step of a partial sum takes a level at a time, as the accumulators are read out.  The others
-            // take a plane of A at a time, against as many planes of B in one MMA as 256 columns hold: an MMA of 64
-            // columns reads 4 KB of A and 2 KB of B in its 32 clocks, more than shared memory gives beside the
-            // loads.  complex128: 10 MMAs and 96 KB per 16 K' instead of 28 and 168 KB, complex64: 4 and 40 KB instead
-            // of 6 and 48 KB.  Exact sums may be taken in any order.
-            constexpr int G = 256 / S::BN;
-            auto row = [&](auto plane, int kk) {
-                constexpr int P = decltype(plane)::value, CNT = S::LV - P;
-                mma(std::integral_constant<int, (CNT < G ? CNT : G)>{}, P, 0, P, kk, false);
-                if constexpr (CNT > G) mma(std::integral_constant<int, CNT - G>{}, P, G, P + G, kk, false);
-            };
-            static_assert(S::LV <= 2 * G, "two MMAs at most for each plane of A");
+            if constexpr (S::LV == 1) {
+                // one accumulator: the small products h l and l h first, while the sum is small and is truncated little
+                static_assert(S::CT == 1 && S::SETS % S::PPS == 0, "whole partial sums per stage");
+                constexpr int KH = S::BK / 16 / S::PPS;
 #pragma unroll
-            for (int kk = 0; kk < S::BK / 16; ++kk) {
-                const bool end = kk == S::BK / 16 - 1 && last;
-                if (kk == 0 && first) {
+                for (int h = 0; h < S::PPS; ++h) {
+                    if (use > 0) drained(h);
 #pragma unroll
-                    for (int l = 0; l < S::LV; ++l) {
-                        if (part > 0) drained(l);
-#pragma unroll
-                        for (int p = 0; p <= l; ++p) mma(one{}, p, l - p, l, kk, p == 0);
-                        if (end && leader) ptx::umma_commit(bar_ready(l));
+                    for (int kk = h * KH; kk < (h + 1) * KH; ++kk) {
+                        mma(one{}, 0, 1, h, kk, kk == h * KH);
+                        mma(one{}, 1, 0, h, kk, false);
                     }
-                } else {
-                    auto plane = [&](auto p) {  // with it the level of its own index has all its products
-                        row(p, kk);
-                        if (end && leader) ptx::umma_commit(bar_ready(decltype(p)::value));
-                    };
-                    each_level<S::LV>(plane);
+#pragma unroll
+                    for (int kk = h * KH; kk < (h + 1) * KH; ++kk) mma(one{}, 0, 0, h, kk, false);
+                    if (leader) ptx::umma_commit(bar_ready(set + h));
+                }
+            } else {
+                // The first step of a partial sum takes a level at a time, as the accumulators are read out.  The others
+                // take a plane of A at a time, against as many planes of B in one MMA as 256 columns hold: an MMA of 64
+                // columns reads 4 KB of A and 2 KB of B in its 32 clocks, more than shared memory gives beside the
+                // loads.  complex128: 10 MMAs and 96 KB per 16 K' instead of 28 and 168 KB, complex64: 4 and 40 KB instead
+                // of 6 and 48 KB.  Exact sums may be taken in any order.
+                constexpr int G = 256 / S::BN;
+                auto row = [&](auto plane, int kk) {
+                    constexpr int P = decltype(plane)::value, CNT = S::LV - P;
+                    mma(std::integral_constant<int, (CNT < G ? CNT : G)>{}, P, 0, P, kk, false);
+                    if constexpr (CNT > G) mma(std::integral_constant<int, CNT - G>{}, P, G, P + G, kk, false);
+                };
+                static_assert(S::LV <= 2 * G, "two MMAs at most for each plane of A");
+#pragma unroll
+                for (int kk = 0; kk < S::BK / 16; ++kk) {
+                    const bool end = kk == S::BK / 16 - 1 && last;
+                    if (kk == 0 && first) {
+#pragma unroll
+                        for (int l = 0; l < S::LV; ++l) {
+                            if (use > 0) drained(l);
+#pragma unroll
+                            for (int p = 0; p <= l; ++p) mma(one{}, p, l - p, l, kk, p == 0);
+                            if (end && leader) ptx::umma_commit(bar_ready(set * S::LV + l));
+                        }
+                    } else {
+                        auto plane = [&](auto p) {  // with it the level of its own index has all its products
+                            row(p, kk);
+                            if (end && leader) ptx::umma_commit(bar_ready(set * S::LV + decltype(p)::value));
+                        };
+                        each_level<S::LV>(plane);
+                    }
                 }
             }
             if (leader) ptx::umma_commit(bar_empty(s));
@@ -526,15 +609,17 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     // of a K split: the partial sums of the tile's CTAs, [CTA][complex column][re, im][row]
     Acc* others = g.parts + ((long long)blockIdx.y * g.n_tiles + n_tile) * KS * (LY::TN * 2 * BM);
     if (epi) {
-        Sums<T> sums;
-        sums.clear();
+        Sums<F> sums;
+        sums.start(g.ktiles * S::PPS / 2, kt0 * S::PPS);  // partial sums per half of K', and the first one's index
         bool live = true;
-        const int nparts = (nkt + S::CT - 1) / S::CT;
+        const int nparts = (nkt + S::CT - 1) / S::CT * S::PPS;
 #pragma unroll 1
         for (int p = 0; p < nparts; ++p) {
+            const int set = p % S::SETS, ph = (p / S::SETS) & 1;
             auto level = [&](auto lc) {
                 constexpr int l = decltype(lc)::value;
-                if (live && !ptx::mbar_wait_bounded(bar_ready(l), p & 1, g.wait_limit)) give_up();
+                const int a = set * S::LV + l;
+                if (live && !ptx::mbar_wait_bounded(bar_ready(a), ph, g.wait_limit)) give_up();
                 // warp-uniform: the TMEM loads are .sync.aligned
                 live = __shfl_sync(0xffffffffu, (int)(live && *abort_flag == 0), 0) != 0;
                 if (!live) return;
@@ -542,15 +627,16 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
 #pragma unroll
                 for (int j0 = 0; j0 < COLS; j0 += LY::LD) {
                     float v[LY::LD];
-                    tmem_ld<LY::LD>(tmem + lane_base + l * S::BN + slice * COLS + j0, v);
+                    tmem_ld<LY::LD>(tmem + lane_base + a * S::BN + slice * COLS + j0, v);
                     sums.template add<l>(j0, v);
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar_drained(l));
+                if (lane == 0) ptx::mbar_arrive(bar_drained(a));
             };
             each_level<S::LV>(level);
             if (!live) break;
+            sums.end_partial(p == nparts - 1);
         }
         // every warp has seen the last accumulators, so this CTA's copies and MMAs are complete
         ptx::named_barrier(1, S::EPI);
@@ -580,11 +666,11 @@ __global__ void __launch_bounds__(Layout<T>::THREADS, 1) plane_gemm_kernel(const
     }
     if (epi) {
         if (KS == 1) ptx::named_barrier(1, S::EPI);
-        if (*abort_flag) rs = NAN_EXP;  // sums that are not complete: every result of theirs is NaN
-        if (KS == 1) finish_columns<T, 1>(g, part_s, others, s_cs, rs, m0, n_tile, 0, et);
-        else if (KS == 2) finish_columns<T, 2>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
-        else if (KS == 4) finish_columns<T, 4>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
-        else finish_columns<T, 8>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+        if (*abort_flag) rs = S::poison();  // sums that are not complete: every result of theirs is NaN
+        if (KS == 1) finish_columns<F, 1>(g, part_s, others, s_cs, rs, m0, n_tile, 0, et);
+        else if (KS == 2) finish_columns<F, 2>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+        else if (KS == 4) finish_columns<F, 4>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
+        else finish_columns<F, 8>(g, part_s, others, s_cs, rs, m0, n_tile, ks, et);
     }
     ptx::tc_fence_before();
     __syncthreads();

@@ -26,7 +26,17 @@ namespace {
 
 // ---- cutting values into planes -----------------------------------------------------------------------------
 
-// Exponent E with |x| <= 2^E for every |x| whose bit pattern is at most mx.
+// Floating planes: power of two s with |x| / s <= 2^15 for every |x| <= mx.  The fp16 value h of x / s then leaves room for a
+// second one of the same weight, x / s - h, whose 11 bits are normal down to 2^-18 of the row's maximum.  s and 1 / s are
+// normal floats, and a row below 2^-111 keeps every bit of its subnormal values.
+__device__ __forceinline__ float plane_scale(float mx) {
+    if (!(mx > 0.0f)) return 1.0f;
+    int e = 128;  // infinities: the planes then hold infinities and NaNs
+    if (isfinite(mx)) frexpf(mx, &e);
+    return ldexpf(1.0f, max(e, -111) - 15);
+}
+
+// Digits: exponent E with |x| <= 2^E for every |x| whose bit pattern is at most mx.
 __device__ __forceinline__ int plane_exponent(unsigned long long mx) {
     const int e = (int)(mx >> 52);
     if (e == 0x7ff) return NAN_EXP;
@@ -58,10 +68,24 @@ __device__ __forceinline__ long long to_fixed(double x, int E) {
     return (b >> 63) ? -(long long)q : (long long)q;
 }
 
-// The planes of four consecutive real values: out[p] holds them as four halves.  x 2^(26 - E) is an integer of 27 bits in
+// The planes of four consecutive real values: out[p] holds them as four halves.
+__device__ __forceinline__ void cut4(C64Floats, const float* x, float inv, uint2* out) {
+    __half2 h[2], l[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const float a = x[2 * q] * inv, b = x[2 * q + 1] * inv;
+        h[q] = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(h[q]);
+        l[q] = __floats2half2_rn(a - f.x, b - f.y);
+    }
+    out[0] = make_uint2(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]));
+    out[1] = make_uint2(*reinterpret_cast<uint32_t*>(&l[0]), *reinterpret_cast<uint32_t*>(&l[1]));
+}
+
+// x 2^(26 - E) is an integer of 27 bits in
 // digits of 9 (two exact steps, since 2^(26 - E) itself may be out of range); with 256 added to each digit, bits 0-8
 // are plane 2, 9-17 plane 1 and what is left plane 0.
-__device__ __forceinline__ void cut4(const float* x, int E, uint2* out) {
+__device__ __forceinline__ void cut4(C64Digits, const float* x, int E, uint2* out) {
     const int k = E == NAN_EXP ? 0 : 26 - E, k1 = min(k, 120);
     const float f1 = __int_as_float((k1 + 127) << 23), f2 = __int_as_float((k - k1 + 127) << 23);
     uint32_t q[4];
@@ -83,7 +107,7 @@ __device__ __forceinline__ void cut4(const float* x, int E, uint2* out) {
     }
 }
 
-__device__ __forceinline__ void cut4(const double* x, int E, uint2* out) {
+__device__ __forceinline__ void cut4(C128Digits, const double* x, int E, uint2* out) {
     unsigned long long q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)  // each digit + 128: bytes 0-5 are planes 6-1, what is left of byte 6 up plane 0
@@ -114,6 +138,14 @@ template <> struct MaxBits<double> {
     using V = unsigned long long;
     __device__ static V of(double x) { return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull; }
 };
+
+// The scale of a row from the bit pattern of its maximum, and what cut4 takes of it.
+__device__ __forceinline__ float row_scale(C64Floats, unsigned int m) {
+    return plane_scale(__uint_as_float(min(m, 0x7f800000u)));
+}
+template <typename F, typename V> __device__ __forceinline__ int row_scale(F, V m) { return plane_exponent(m); }
+__device__ __forceinline__ float cut_factor(float s) { return 1.0f / s; }
+__device__ __forceinline__ int cut_factor(int e) { return e; }
 
 template <typename V> __device__ __forceinline__ V block_max(V m, V* red) {
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -147,16 +179,18 @@ __device__ __forceinline__ void load4(const double2* p, int k0, int K, double* r
 
 // One CTA per row of K complex values: the row's scale, and its planes [Re | Im], each Kp long with zeros past K.
 // Four values per thread and step, kept in registers between the maximum and the cut up to G steps (a longer row is
-// read twice), so the pass is bound by the bytes it moves: 8 B in and 12 B out per complex64 value, 16 and 28 B per
+// read twice), so the pass is bound by the bytes it moves: 8 B in and 12 B (8 B) out per complex64 value, 16 and 28 B per
 // complex128 value.  W: value k of a row is multiplied by wk[k].
-template <typename T, int G, bool W>
-__global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>::type* __restrict__ in, long long ld,
-                                                         int K, int Kp, const T* __restrict__ wk,
+template <typename F, int G, bool W>
+__global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<typename Shape<F>::T>::type* __restrict__ in,
+                                                         long long ld, int K, int Kp,
+                                                         const typename Shape<F>::T* __restrict__ wk,
                                                          __half* __restrict__ planes, long long plane_stride,
                                                          int kpitch,
-                                                         typename Shape<T>::Scale* __restrict__ scale_out) {
+                                                         typename Shape<F>::Scale* __restrict__ scale_out) {
+    using T = typename Shape<F>::T;
     using MB = MaxBits<T>;
-    constexpr int NP = Shape<T>::NP;
+    constexpr int NP = Shape<F>::NP;
     __shared__ typename MB::V red[8];
     auto load = [&](const typename cplx<T>::type* p, int k0, T* a, T* b) {
         load4(p, k0, K, a, b);
@@ -186,12 +220,13 @@ __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>:
 #pragma unroll
         for (int j = 0; j < 4; ++j) mx = max(mx, max(MB::of(a[j]), MB::of(b[j])));
     }
-    const int f = plane_exponent(block_max(mx, red));
-    if (threadIdx.x == 0) scale_out[m] = f;
+    const auto s = row_scale(F(), block_max(mx, red));
+    if (threadIdx.x == 0) scale_out[m] = s;
+    const auto f = cut_factor(s);
     auto put = [&](int k0, const T* a, const T* b) {
         uint2 cr[NP], ci[NP];
-        cut4(a, f, cr);
-        cut4(b, f, ci);
+        cut4(F(), a, f, cr);
+        cut4(F(), b, f, ci);
         __half* dst = planes + m * kpitch + k0;
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
@@ -213,18 +248,20 @@ __global__ void __launch_bounds__(256) plane_rows_kernel(const typename cplx<T>:
 
 // One CTA per column n of a constant operand V[n][k] = wn[n] exp(sign i a[n] b[k]), evaluated in float64 as the phase
 // matrices of the CUDA-core form are: the rows [Re | -Im] and [Im | Re] of its embedding.
-template <typename T>
+template <typename F>
 __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const double* __restrict__ a,
                                                           const double* __restrict__ b, double sign,
                                                           const double* __restrict__ wn, __half* __restrict__ planes,
                                                           long long plane_stride, int kpitch,
-                                                          typename Shape<T>::Scale* __restrict__ scale_out) {
+                                                          typename Shape<F>::Scale* __restrict__ scale_out) {
+    using T = typename Shape<F>::T;
     using MB = MaxBits<T>;
-    constexpr int NP = Shape<T>::NP;
+    constexpr int NP = Shape<F>::NP;
     const int n = blockIdx.x;
     const double w = wn ? wn[n] : 1.0;
-    const int f = plane_exponent(MB::of((T)w));  // both parts are at most |w|
-    if (threadIdx.x == 0) scale_out[n] = f;
+    const auto s = row_scale(F(), MB::of((T)w));  // both parts are at most |w|
+    if (threadIdx.x == 0) scale_out[n] = s;
+    const auto f = cut_factor(s);
     const long long r_re = (long long)(n >> 3) * 16 + (n & 7), r_im = r_re + 8;
     for (int k0 = 4 * threadIdx.x; k0 < Kp; k0 += 4 * blockDim.x) {
         T re[4], im[4], ni[4];
@@ -242,9 +279,9 @@ __global__ void __launch_bounds__(256) plane_const_kernel(int K, int Kp, const d
             ni[j] = -im[j];
         }
         uint2 cr[NP], ci[NP], cn[NP];
-        cut4(re, f, cr);
-        cut4(im, f, ci);
-        cut4(ni, f, cn);
+        cut4(F(), re, f, cr);
+        cut4(F(), im, f, ci);
+        cut4(F(), ni, f, cn);
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             __half* pl = planes + p * plane_stride;
@@ -286,6 +323,7 @@ struct PlaneMat {
     long long rows = 0;
     int K = 0, Kp = 0, kpitch = 0;
     int n = 0;  // complex columns of a constant operand
+    bool digits = true;
     CUtensorMap map;  // of a constant operand, encoded once
     long long plane_stride() const { return rows * kpitch; }
 };
@@ -302,28 +340,44 @@ struct Carver {
     }
 };
 
-template <typename T> void carve_mat(Carver& c, PlaneMat& m, long long rows, long long scales, int K) {
+// The form of complex64 operands, from the length K of the sum and the longest side of the two grids.  Floating planes take
+// half the products of digits (three fields back from 165^2 to 1001^2 points 65 against 74 us, a Lyot pass over four
+// 1024^2 fields 333 against 434), but what their truncated sums lose adds up along a chain of transforms, beside the CUDA
+// cores' error, which grows with the sums.  Gradients through a Lyot coronagraph and an image (512^2 and 256^2 points,
+// twelve GEMMs) from 512^2, 700^2 and 1024^2 pupils are off by
+//   digits 0.9, 0.9 and 1.2e-7, floating planes 3.9, 3.8 and 3.7e-7, CUDA cores 3.4, 3.3 and 4.6e-7,
+// so floating planes take over between the last two.  Short sums always take digits: a sum of few partial sums has no
+// mean loss to take back (see Sums<C64Floats>), and the GEMM is not bound by its products.
+inline bool takes_digits(int K, int longest) { return longest <= 960 || K <= 128; }
+
+// fn with the form as a value of its type.
+template <typename T, typename Fn> auto with_form(bool digits, Fn&& fn) {
+    if constexpr (sizeof(T) == 8) return fn(C128Digits());
+    else return digits ? fn(C64Digits()) : fn(C64Floats());
+}
+
+template <typename F> void carve_mat(Carver& c, PlaneMat& m, long long rows, long long scales, int K) {
     m.K = K;
     m.Kp = (int)round_up(K, 32);
     m.kpitch = 2 * m.Kp;
     m.rows = rows;
-    m.planes = (__half*)c.take(sizeof(__half) * Shape<T>::NP * (size_t)rows * m.kpitch);
-    m.scale = c.take(sizeof(typename Shape<T>::Scale) * (size_t)scales);
+    m.planes = (__half*)c.take(sizeof(__half) * Shape<F>::NP * (size_t)rows * m.kpitch);
+    m.scale = c.take(sizeof(typename Shape<F>::Scale) * (size_t)scales);
 }
 
-template <typename T> int encode_map(CUtensorMap* map, const PlaneMat& m, int box_rows) {
+template <typename F> int encode_map(CUtensorMap* map, const PlaneMat& m, int box_rows) {
     auto enc = get_encode();
     if (!enc) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
         return HX_ERR_UNSUPPORTED;
     }
-    cuuint64_t dims[3] = {(cuuint64_t)m.kpitch, (cuuint64_t)m.rows, (cuuint64_t)Shape<T>::NP};
+    cuuint64_t dims[3] = {(cuuint64_t)m.kpitch, (cuuint64_t)m.rows, (cuuint64_t)Shape<F>::NP};
     cuuint64_t strides[2] = {(cuuint64_t)m.kpitch * 2, (cuuint64_t)m.rows * m.kpitch * 2};
-    cuuint32_t box[3] = {(cuuint32_t)Shape<T>::BK, (cuuint32_t)box_rows, (cuuint32_t)Shape<T>::NP};
+    cuuint32_t box[3] = {(cuuint32_t)Shape<F>::BK, (cuuint32_t)box_rows, (cuuint32_t)Shape<F>::NP};
     cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, m.planes, dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           Layout<T>::ROW_BYTES == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           Layout<F>::ROW_BYTES == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled failed (%d) for %lld rows x %d", (int)r, m.rows, m.kpitch);
@@ -332,15 +386,16 @@ template <typename T> int encode_map(CUtensorMap* map, const PlaneMat& m, int bo
     return HX_OK;
 }
 
-template <typename T>
+template <typename F>
 int launch_rows(const void* in, long long rows, int K, const void* wk, const PlaneMat& m, cudaStream_t st) {
+    using T = typename Shape<F>::T;
     using Cx = typename cplx<T>::type;
-    using Sc = typename Shape<T>::Scale;
+    using Sc = typename Shape<F>::Scale;
     const int threads = std::min<int>(256, (int)round_up((m.Kp + 3) / 4, 32));
     const int steps = (m.Kp + 4 * threads - 1) / (4 * threads);
     const unsigned grid = (unsigned)rows;
     auto run = [&](auto g, auto weighted) {
-        plane_rows_kernel<T, decltype(g)::value, decltype(weighted)::value><<<grid, threads, 0, st>>>(
+        plane_rows_kernel<F, decltype(g)::value, decltype(weighted)::value><<<grid, threads, 0, st>>>(
             (const Cx*)in, K, K, m.Kp, (const T*)wk, m.planes, m.plane_stride(), m.kpitch, (Sc*)m.scale);
     };
     if (wk) run(std::integral_constant<int, 1>(), std::true_type());
@@ -351,7 +406,7 @@ int launch_rows(const void* in, long long rows, int K, const void* wk, const Pla
 }
 
 // Whether clusters of ks CTAs of the GEMM can be resident on this device.
-template <typename T> bool cluster_ok(int ks) {
+template <typename F> bool cluster_ok(int ks) {
     static int cache[64][9];  // per device: 0 unknown, 1 yes, 2 no
     static const bool off = [] {  // HX_NO_CLUSTERS=1: no K split (tests of that path)
         const char* e = getenv("HX_NO_CLUSTERS");
@@ -362,8 +417,8 @@ template <typename T> bool cluster_ok(int ks) {
     if (!cache[dev][ks]) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ks);
-        cfg.blockDim = dim3(Layout<T>::THREADS);
-        cfg.dynamicSmemBytes = Layout<T>::SMEM;
+        cfg.blockDim = dim3(Layout<F>::THREADS);
+        cfg.dynamicSmemBytes = Layout<F>::SMEM;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)ks;
@@ -372,35 +427,36 @@ template <typename T> bool cluster_ok(int ks) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        const bool ok = cudaFuncSetAttribute(plane_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             Layout<T>::SMEM) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&n, plane_gemm_kernel<T>, &cfg) == cudaSuccess && n > 0;
+        const bool ok = cudaFuncSetAttribute(plane_gemm_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             Layout<F>::SMEM) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, plane_gemm_kernel<F>, &cfg) == cudaSuccess && n > 0;
         cudaGetLastError();
         cache[dev][ks] = ok ? 1 : 2;
     }
     return cache[dev][ks] == 1;
 }
 
-// CTAs along K per tile: enough to occupy the SMs, each with at least one partial sum (256 terms of K' in complex64, 128 in
-// complex128), below which the exchange costs more than the shorter chain saves.
-template <typename T> int k_split(long long tiles, int ktiles, bool throughput) {
+// CTAs along K per tile: enough to occupy the SMs, each with at least 256 terms of K' (128 in complex128), below which the
+// exchange costs more than the shorter chain saves.
+template <typename F> int k_split(long long tiles, int ktiles, bool throughput) {
     if (throughput) return 1;
-    const int parts = (ktiles + Shape<T>::CT - 1) / Shape<T>::CT;
+    const int parts = (ktiles + Shape<F>::CT - 1) / Shape<F>::CT;
+    constexpr int least = std::is_same<F, C64Floats>::value ? 4 : 1;
     for (int ks : {8, 4, 2})
-        if (tiles * ks <= num_sms() && parts / ks >= 1 && cluster_ok<T>(ks)) return ks;
+        if (tiles * ks <= num_sms() && parts / ks >= least && cluster_ok<F>(ks)) return ks;
     return 1;
 }
 
-template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const PlaneMat& b, bool throughput,
+template <typename F> int launch_gemm(PlaneArgs<F>& g, const PlaneMat& a, const PlaneMat& b, bool throughput,
                                       double cmacs, cudaStream_t st) {
-    using LY = Layout<T>;
-    HX_TRY(encode_map<T>(&g.tmap_a, a, BM));
+    using LY = Layout<F>;
+    HX_TRY(encode_map<F>(&g.tmap_a, a, BM));
     g.tmap_b = b.map;
     static bool configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        HX_TRY(cuda_status(cudaFuncSetAttribute(plane_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HX_TRY(cuda_status(cudaFuncSetAttribute(plane_gemm_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 LY::SMEM),
                            "cudaFuncSetAttribute(plane_gemm_kernel)"));
         if (dev >= 0 && dev < 64) configured[dev] = true;
@@ -408,18 +464,18 @@ template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const 
     g.M = (int)a.rows;
     g.N = b.n;
     g.alpha_kind = g.alpha.y == 0 ? (g.alpha.x == 1 ? 0 : 1) : g.alpha.x == 0 ? 2 : 3;
-    g.row_scale = (const typename Shape<T>::Scale*)a.scale;
-    g.col_scale = (const typename Shape<T>::Scale*)b.scale;
-    g.ktiles = a.kpitch / Shape<T>::BK;
+    g.row_scale = (const typename Shape<F>::Scale*)a.scale;
+    g.col_scale = (const typename Shape<F>::Scale*)b.scale;
+    g.ktiles = a.kpitch / Shape<F>::BK;
     g.stall = fault_injected("wait");
     g.wait_limit = g.stall ? 10000000ull : WAIT_LIMIT;
     g.n_tiles = (int)ceil_div(b.n, LY::TN);
     const unsigned m_tiles = ceil_div(a.rows, BM);
-    g.ksplit = k_split<T>((long long)m_tiles * g.n_tiles, g.ktiles, throughput);
+    g.ksplit = k_split<F>((long long)m_tiles * g.n_tiles, g.ktiles, throughput);
     TraceScope trace(HX_TRACE_SIMT_GEMM, cmacs, st);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(g.n_tiles * g.ksplit), m_tiles);
-    cfg.blockDim = dim3(Layout<T>::THREADS);
+    cfg.blockDim = dim3(Layout<F>::THREADS);
     cfg.dynamicSmemBytes = LY::SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -429,7 +485,7 @@ template <typename T> int launch_gemm(PlaneArgs<T>& g, const PlaneMat& a, const 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g.ksplit > 1 ? 1 : 0;
-    HX_TRY(cuda_status(cudaLaunchKernelEx(&cfg, plane_gemm_kernel<T>, g), "plane_gemm_kernel"));
+    HX_TRY(cuda_status(cudaLaunchKernelEx(&cfg, plane_gemm_kernel<F>, g), "plane_gemm_kernel"));
     return launch_status("plane_gemm_kernel");
 }
 
@@ -449,6 +505,7 @@ namespace {
 // The source plane (K1 x K2) and the destination plane (R x C) of a direction.
 struct Dims {
     int K1, K2, R, C;
+    int longest() const { return std::max(std::max(K1, K2), std::max(R, C)); }
 };
 Dims dims_of(const PlaneMft* p, int direction) {
     if (direction == HX_FORWARD) return {p->ny, p->nx, p->nv, p->nu};
@@ -468,13 +525,20 @@ template <typename T> size_t carve_pass(void* ws, const Dims& d, int fields, Pas
     Carver c((void*)(((uintptr_t)ws + 255) / 256 * 256));  // TMA wants 16 bytes; a caller's scratch may start anywhere
     Pass<T> q;
     const long long r1 = (long long)fields * d.K1, r2 = (long long)fields * d.C;
-    carve_mat<T>(c, q.s1, r1, r1, d.K2);
+    auto mat = [&](PlaneMat& m, long long rows, int K) {
+        m.digits = takes_digits(K, d.longest());
+        with_form<T>(m.digits, [&](auto f) { carve_mat<decltype(f)>(c, m, rows, rows, K); });
+    };
+    mat(q.s1, r1, d.K2);
     q.t = c.take(2 * sizeof(T) * (size_t)r2 * d.K1);
-    carve_mat<T>(c, q.s2, r2, r2, d.K1);
+    mat(q.s2, r2, d.K1);
     auto part_bytes = [&](const PlaneMat& a, int N) {
-        const long long tiles = (long long)ceil_div(a.rows, BM) * ceil_div(N, Layout<T>::TN);
-        const int ks = k_split<T>(tiles, a.kpitch / Shape<T>::BK, false);
-        return ks > 1 ? (size_t)tiles * ks * Layout<T>::TN * 2 * BM * sizeof(typename Shape<T>::Acc) : (size_t)0;
+        return with_form<T>(a.digits, [&](auto f) {
+            using F = decltype(f);
+            const long long tiles = (long long)ceil_div(a.rows, BM) * ceil_div(N, Layout<F>::TN);
+            const int ks = k_split<F>(tiles, a.kpitch / Shape<F>::BK, false);
+            return ks > 1 ? (size_t)tiles * ks * Layout<F>::TN * 2 * BM * sizeof(typename Shape<F>::Acc) : (size_t)0;
+        });
     };
     q.parts = c.take(std::max(part_bytes(q.s1, d.C), part_bytes(q.s2, d.R)));
     q.bytes = c.off + 255;
@@ -505,10 +569,13 @@ template <typename T> int make_const(PlaneMat& m, int N, const double* a, const 
                                      const double* wn, cudaStream_t st) {
     m.n = N;
     if (fault_injected("operand_map")) return HX_ERR_INJECTED;
-    HX_TRY(encode_map<T>(&m.map, m, Shape<T>::BN));
-    plane_const_kernel<T><<<(unsigned)N, 256, 0, st>>>(m.K, m.Kp, a, b, sign, wn, m.planes, m.plane_stride(),
-                                                       m.kpitch, (typename Shape<T>::Scale*)m.scale);
-    return launch_status("plane_const_kernel");
+    return with_form<T>(m.digits, [&](auto f) {
+        using F = decltype(f);
+        HX_TRY(encode_map<F>(&m.map, m, Shape<F>::BN));
+        plane_const_kernel<F><<<(unsigned)N, 256, 0, st>>>(m.K, m.Kp, a, b, sign, wn, m.planes, m.plane_stride(), m.kpitch,
+                                                           (typename Shape<F>::Scale*)m.scale);
+        return launch_status("plane_const_kernel");
+    });
 }
 
 template <typename T>
@@ -518,8 +585,12 @@ int create_t(PlaneMft* p, const double* x, const double* y, const double* u, con
     auto layout = [&](Carver& c) {
         for (int d = 0; d < (own_adjoint ? 3 : 2); ++d) {
             const Dims q = dims_of(p, d);
-            carve_mat<T>(c, p->rgt[d], 2 * round_up(q.C, 8), q.C, q.K2);
-            carve_mat<T>(c, p->lft[d], 2 * round_up(q.R, 8), q.R, q.K1);
+            auto mat = [&](PlaneMat& m, int columns, int K) {
+                m.digits = takes_digits(K, q.longest());
+                with_form<T>(m.digits, [&](auto f) { carve_mat<decltype(f)>(c, m, 2 * round_up(columns, 8), columns, K); });
+            };
+            mat(p->rgt[d], q.C, q.K2);
+            mat(p->lft[d], q.R, q.K1);
         }
         auto weights = [&](const double* w, int n) { return w ? c.take(sizeof(T) * (size_t)n) : nullptr; };
         p->wk2[HX_FORWARD] = weights(wx, p->nx);
@@ -576,34 +647,41 @@ int execute_t(const PlaneMft* p, int direction, int batch, const void* in, void*
         const int b0 = (grow ? passes - 1 - i : i) * per, nb = std::min(per, batch - b0);
         Pass<T> q;
         carve_pass<T>(ws, d, nb, &q);
-        const Cx* src_f = (const Cx*)in + (long long)b0 * d.K1 * d.K2;
         const long long oplane = (long long)d.R * d.C;
-        HX_TRY(launch_rows<T>(src_f, (long long)nb * d.K1, d.K2, p->wk2[direction], q.s1, st));
-        PlaneArgs<T> g1;
-        memset(&g1, 0, sizeof(g1));
-        g1.rows_per_field = d.K1;
-        g1.ldo = d.K1;
-        g1.out_z = (long long)d.C * d.K1;
-        g1.out = (Cx*)q.t;
-        g1.alpha = make_c<T>(T(1), T(0));
-        g1.epi = HX_EPI_NONE;
-        g1.parts = (typename Shape<T>::Acc*)q.parts;
-        g1.status = p->status;
-        HX_TRY(launch_gemm<T>(g1, q.s1, p->rgt[direction], throughput, (double)nb * d.K1 * d.K2 * d.C, st));
-        HX_TRY(launch_rows<T>(q.t, (long long)nb * d.C, d.K1, p->wk1[direction], q.s2, st));
-        PlaneArgs<T> g2;
-        memset(&g2, 0, sizeof(g2));
-        g2.rows_per_field = d.C;
-        g2.ldo = d.C;
-        g2.out_z = oplane;
-        g2.out = (Cx*)out + b0 * oplane;
-        g2.alpha = make_c<T>((T)are, (T)aim);
-        g2.epi = epilogue;
-        g2.mask = (const Cx*)mask;
-        g2.src = src ? (const Cx*)src + b0 * oplane : nullptr;
-        g2.parts = (typename Shape<T>::Acc*)q.parts;
-        g2.status = p->status;
-        HX_TRY(launch_gemm<T>(g2, q.s2, p->lft[direction], throughput, (double)nb * d.R * d.K1 * d.C, st));
+        // cut the rows of `from`, then multiply them with a constant
+        auto product = [&](const void* from, long long rows, const void* wk, const PlaneMat& a, const PlaneMat& b,
+                           double cmacs, auto&& set) {
+            return with_form<T>(a.digits, [&](auto f) {
+                using F = decltype(f);
+                HX_TRY(launch_rows<F>(from, rows, a.K, wk, a, st));
+                PlaneArgs<F> g;
+                memset(&g, 0, sizeof(g));
+                g.parts = (typename Shape<F>::Acc*)q.parts;
+                g.status = p->status;
+                set(g);
+                return launch_gemm<F>(g, a, b, throughput, cmacs, st);
+            });
+        };
+        HX_TRY(product((const Cx*)in + (long long)b0 * d.K1 * d.K2, (long long)nb * d.K1, p->wk2[direction], q.s1,
+                       p->rgt[direction], (double)nb * d.K1 * d.K2 * d.C, [&](auto& g) {
+                           g.rows_per_field = d.K1;
+                           g.ldo = d.K1;
+                           g.out_z = (long long)d.C * d.K1;
+                           g.out = (Cx*)q.t;
+                           g.alpha = make_c<T>(T(1), T(0));
+                           g.epi = HX_EPI_NONE;
+                       }));
+        HX_TRY(product(q.t, (long long)nb * d.C, p->wk1[direction], q.s2, p->lft[direction],
+                       (double)nb * d.R * d.K1 * d.C, [&](auto& g) {
+                           g.rows_per_field = d.C;
+                           g.ldo = d.C;
+                           g.out_z = oplane;
+                           g.out = (Cx*)out + b0 * oplane;
+                           g.alpha = make_c<T>((T)are, (T)aim);
+                           g.epi = epilogue;
+                           g.mask = (const Cx*)mask;
+                           g.src = src ? (const Cx*)src + b0 * oplane : nullptr;
+                       }));
     }
     return HX_OK;
 }
@@ -615,7 +693,7 @@ bool plane_mft_fits(int nx, int ny, int nu, int nv, int dtype, bool weighted) {
     if (std::min(std::min(nx, ny), std::min(nu, nv)) < 16) return false;
     // The operands of the two directions, and of the adjoint where weights make it a third: at most 8 GB, 3% of the memory
     // (complex64 transforms between uniform grids of 8192^2 points take 6.4).
-    const double bytes = 8.0 * (dtype == HX_C64 ? Shape<float>::NP : Shape<double>::NP) * (weighted ? 3.0 : 2.0) *
+    const double bytes = 8.0 * (dtype == HX_C64 ? Shape<C64Digits>::NP : Shape<C128Digits>::NP) * (weighted ? 3.0 : 2.0) *
                          ((double)nx * nu + (double)ny * nv);
     return bytes <= 8e9;
 }
