@@ -7,8 +7,9 @@
 //
 // Operands.  Every row of A and of B is scaled by a power of two and cut into fp16 planes, in one of three forms (plane_mft.cu
 // says which a complex64 operand takes):
-//   C64Digits : x = 2^E sum_i d_i 2^(-8 - 9 i) with |x| <= 2^E, three digits of base 512, d_i in [-256, 256], to 2^-27 of 2^E;
-//               the six products d_i d_j with i + j <= 2 go to three accumulators, one per level i + j;
+//   C64Digits : x = 2^E sum_i d_i 2^(-8 - 9 i) with |x| <= 2^E, two whole digits of base 512, d_i in [-256, 256], and the rest
+//               as an fp16 value: exact for |x| >= 2^(E - 6), to 2^-30 of 2^E below; the six products d_i d_j with
+//               i + j <= 2 go to three accumulators, one per level i + j;
 //   C64Floats : x = s (h + l), h and l the fp16 roundings of x / s and of x / s - h, which keeps 22 bits of every element;
 //               the products h l, l h and h h go to one FP32 accumulator, the small ones first;
 //   C128Digits: x = 2^E sum_i d_i 2^(-7 - 8 i), seven digits of base 256, d_i in [-128, 128], to 2^-56 of 2^E; the 28
@@ -29,8 +30,9 @@
 //   C128Digits: 128 terms: every level is below 7 * 128 * 2^14 < 2^24, hence exact, and is added to 64-bit integers
 //               (levels 0-3 in one, 4-6 in another), exact over any K the plans take.
 // The error of a transform in digits is that of its operands (above), of the dropped products (of digits 1 and 2 in complex64:
-// 2^-26 of the two scales at most) and one rounding of each sum: 3.5-7.5e-8 in complex64.  In floating planes it is
-// 1.1-2.0e-7, where the CUDA cores' sums of as many terms are 5e-7 to 1.6e-6 off.
+// 2^-26 of the two scales at most, 2.5e-9 in the mean square) and one rounding of each sum: 3.5-7e-8 in complex64, for fields
+// whose brightest pixel is 1e3 to 1e7 times the others 1.0-5.2e-7 (96 to 960 terms; CUDA cores 3.5e-7 to 1.7e-6).  In
+// floating planes it is 1.1-2.0e-7, where the CUDA cores' sums of as many terms are 5e-7 to 1.6e-6 off.
 //
 // Pipeline.  One CTA per 128 rows x BN real columns (BN = 128 for complex64, 64 for complex128, whose seven levels
 // take 448 of the 512 TMEM columns): warp 0 issues TMA boxes of all planes of a K step, warp 1 the MMAs, the others

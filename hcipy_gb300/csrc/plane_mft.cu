@@ -82,29 +82,37 @@ __device__ __forceinline__ void cut4(C64Floats, const float* x, float inv, uint2
     out[1] = make_uint2(*reinterpret_cast<uint32_t*>(&l[0]), *reinterpret_cast<uint32_t*>(&l[1]));
 }
 
-// x 2^(26 - E) is an integer of 27 bits in
-// digits of 9 (two exact steps, since 2^(26 - E) itself may be out of range); with 256 added to each digit, bits 0-8
-// are plane 2, 9-17 plane 1 and what is left plane 0.
+// v = x 2^(26 - E) (in two exact steps, since 2^(26 - E) itself may be out of range) is 2^9 h and a rest of 256 at most: h, an
+// integer of 18 bits, makes digits 0 and 1 (with 256 added to each, its bits 9 up and 0-8), the rest is digit 2, rounded
+// to the 11 bits of an fp16 value.
 __device__ __forceinline__ void cut4(C64Digits, const float* x, int E, uint2* out) {
     const int k = E == NAN_EXP ? 0 : 26 - E, k1 = min(k, 120);
     const float f1 = __int_as_float((k1 + 127) << 23), f2 = __int_as_float((k - k1 + 127) << 23);
     uint32_t q[4];
+    float r[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = (uint32_t)(E == NAN_EXP ? 0 : __float2int_rn(x[j] * f1 * f2)) + 0x4020100u;
+    for (int j = 0; j < 4; ++j) {
+        const float v = E == NAN_EXP ? 0.0f : x[j] * f1 * f2;
+        const int h = __float2int_rn(v * 0x1p-9f);
+        q[j] = (uint32_t)h + 0x20100u;
+        r[j] = fmaf((float)h, -512.0f, v);
+    }
     const __half2 bias = __halves2half2(__ushort_as_half(0x6500), __ushort_as_half(0x6500));  // 1024 + 256
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
+    for (int p = 0; p < 2; ++p) {
         uint32_t w[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const uint32_t a = p == 0 ? q[2 * i] >> 18 : (q[2 * i] >> (18 - 9 * p)) & 0x1ff;
-            const uint32_t b = p == 0 ? q[2 * i + 1] >> 18 : (q[2 * i + 1] >> (18 - 9 * p)) & 0x1ff;
+            const uint32_t a = p == 0 ? q[2 * i] >> 9 : q[2 * i] & 0x1ff;
+            const uint32_t b = p == 0 ? q[2 * i + 1] >> 9 : q[2 * i + 1] & 0x1ff;
             const uint32_t u = 0x64006400u + (a | (b << 16));  // the halves 1024 + digit + 256
             const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&u), bias);
             w[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
         out[p] = make_uint2(w[0], w[1]);
     }
+    const __half2 l0 = __floats2half2_rn(r[0], r[1]), l1 = __floats2half2_rn(r[2], r[3]);
+    out[2] = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
 }
 
 __device__ __forceinline__ void cut4(C128Digits, const double* x, int E, uint2* out) {

@@ -7,10 +7,11 @@ Operands in digits (grids of up to 960 points a side, and sums of up to 128 term
 rounding, for sums of 16, 32 and 96 terms, of a K' whose halves hold an odd number of 32s, and of many partial sums.
 Tolerance, relative L2 against float64, 1e-7.  A transform rounds three times to 24 bits (the two sums and the product with
 the grid's weight): a rounding is 2^-24 at most, uniform, of a value whose mantissa is spread over its logarithm, 2.5e-8
-in the mean square, so 4.4e-8 together.  The operands, cut at 2^-27 of a row's maximum at most, add 2^-27 / sqrt(3) = 4.3e-9
-of that maximum twice per product, about 2e-8 of random values (maximum 4 to 5 times the mean square), in both products:
-5e-8 in all.  With mantissas that are not spread evenly (all pixels of a smooth field alike) a rounding may be 3.4e-8 in
-the mean square: 7e-8.
+in the mean square, so 4.4e-8 together.  The operands are exact, or cut at 2^-29 of a row's maximum at most, 2^-29 / sqrt(3) =
+1.1e-9 of it in the mean square: 5e-9 of random values.  The products of digits that are left out are 2.5e-9 of the two maxima
+in the mean square: 1.2e-8 of random values.
+With mantissas that are not spread evenly (all pixels of a smooth field alike) a rounding may be 3.4e-8 in
+the mean square: 7e-8 in all.
 Mean error (a factor on the whole transform), 4e-8: roundings to nearest have none for random fields; where
 all sums are alike they share one, 2^-25 = 3e-8 at most in the mean.
 
