@@ -11,9 +11,9 @@
 // The stores go out in pieces of 16 bytes, so the output rows must be aligned to that (stream_fits); others keep
 // split_gemm_kernel, whose warps store element by element along a row.
 //
-// What it measured: GEMMs of 64 stacked fields, 512^2 points to 512^2, complex64-to-float-float 395 -> 296 us, and with
-// complex128 results from 256 points 319 -> 194 us; a gradient step through a Lyot coronagraph over 64 fields of 512^2
-// points 5955 -> 4947 us.  A tile of 16 K steps of 64 takes 36 to 39 thousand clocks, 33 of them MMAs: what is left is the
+// What it measured: GEMMs of 64 stacked fields, 512^2 points to 512^2, complex64-to-float-float 395 -> 298 us, and with
+// complex128 results from 256 points 319 -> 199 us; a gradient step through a Lyot coronagraph over 64 fields of 512^2
+// points 5955 -> 4947 us.  A tile of 16 K steps of 64 takes 37 to 41 thousand clocks, 33 of them MMAs: what is left is the
 // 2 thousand in which the levels are read (TMEM holds one tile's) and loads that the stores delay.
 // On the way there: the loads alone take 23 thousand clocks a tile, so neither they nor L2 bound the loop; the epilogue
 // did, through instructions (see `scale` and store_rows), and through stores that touched 32 lines each.
