@@ -348,15 +348,23 @@ struct Carver {
     }
 };
 
-// The form of complex64 operands, from the length K of the sum and the longest side of the two grids.  Floating planes take
-// half the products of digits (three fields back from 165^2 to 1001^2 points 65 against 74 us, a Lyot pass over four
-// 1024^2 fields 333 against 434), but what their truncated sums lose adds up along a chain of transforms, beside the CUDA
-// cores' error, which grows with the sums.  Gradients through a Lyot coronagraph and an image (512^2 and 256^2 points,
-// twelve GEMMs) from 512^2, 700^2 and 1024^2 pupils are off by
-//   digits 0.9, 0.9 and 1.2e-7, floating planes 3.9, 3.8 and 3.7e-7, CUDA cores 3.4, 3.3 and 4.6e-7,
-// so floating planes take over between the last two.  Short sums always take digits: a sum of few partial sums has no
-// mean loss to take back (see Sums<C64Floats>), and the GEMM is not bound by its products.
-inline bool takes_digits(int K, int longest) { return longest <= 960 || K <= 128; }
+// The form of complex64 operands.  Floating planes take half the products of digits, but what their truncated sums lose adds up
+// along a chain of transforms, beside the CUDA cores' error, which grows with the sums.  Gradients in FP32 through a Lyot
+// coronagraph and an image (512^2 and 256^2 points, six transforms of two products) are off by, in 1e-7:
+//   pupil                  all digits   as below   second products   all floating   CUDA cores
+//   512^2                     0.8         2.9           3.0              4.0           3.5
+//   256^2                     0.9         2.8           4.0              5.3           3.5
+//   400^2                     1.1         2.6           3.0              3.5           2.6
+//   1024^2                    1.2                                        3.7           4.6
+//   (the step, 64 of 512^2)  4.7 ms       4.5           4.2              3.8            13
+// Images of Lyot coronagraphs (511^2 to 700^2 pupils) are off by 1.0-5.9, 5.0-6.8, 5.5-6.6, 7.6-10 and 14-24, and a pass over
+// four 700^2 fields takes 326, 313, 285, 255 and 1022 us.  The plain form is to be as near as the CUDA cores everywhere, at
+// the least time (nearer still is what the split form is for): up to 960 points a side digits in both products of the forward
+// direction and in the second of the others, floating planes beyond.  Short sums take digits always: a sum of few partial
+// sums has no mean loss to take back (see Sums<C64Floats>), and its GEMM is not bound by its products.
+inline bool takes_digits(int K, int longest, int direction, bool second) {
+    return K <= 128 || (longest <= 960 && (second || direction == HX_FORWARD));
+}
 
 // fn with the form as a value of its type.
 template <typename T, typename Fn> auto with_form(bool digits, Fn&& fn) {
@@ -512,12 +520,13 @@ namespace {
 
 // The source plane (K1 x K2) and the destination plane (R x C) of a direction.
 struct Dims {
-    int K1, K2, R, C;
+    int K1, K2, R, C, direction;
     int longest() const { return std::max(std::max(K1, K2), std::max(R, C)); }
+    bool digits(bool second) const { return takes_digits(second ? K1 : K2, longest(), direction, second); }
 };
 Dims dims_of(const PlaneMft* p, int direction) {
-    if (direction == HX_FORWARD) return {p->ny, p->nx, p->nv, p->nu};
-    return {p->nv, p->nu, p->ny, p->nx};
+    if (direction == HX_FORWARD) return {p->ny, p->nx, p->nv, p->nu, direction};
+    return {p->nv, p->nu, p->ny, p->nx, direction};
 }
 
 // Fields per pass: the scratch of a pass stays within 4 GB.
@@ -533,13 +542,13 @@ template <typename T> size_t carve_pass(void* ws, const Dims& d, int fields, Pas
     Carver c((void*)(((uintptr_t)ws + 255) / 256 * 256));  // TMA wants 16 bytes; a caller's scratch may start anywhere
     Pass<T> q;
     const long long r1 = (long long)fields * d.K1, r2 = (long long)fields * d.C;
-    auto mat = [&](PlaneMat& m, long long rows, int K) {
-        m.digits = takes_digits(K, d.longest());
+    auto mat = [&](PlaneMat& m, long long rows, int K, bool digits) {
+        m.digits = digits;
         with_form<T>(m.digits, [&](auto f) { carve_mat<decltype(f)>(c, m, rows, rows, K); });
     };
-    mat(q.s1, r1, d.K2);
+    mat(q.s1, r1, d.K2, d.digits(false));
     q.t = c.take(2 * sizeof(T) * (size_t)r2 * d.K1);
-    mat(q.s2, r2, d.K1);
+    mat(q.s2, r2, d.K1, d.digits(true));
     auto part_bytes = [&](const PlaneMat& a, int N) {
         return with_form<T>(a.digits, [&](auto f) {
             using F = decltype(f);
@@ -593,12 +602,12 @@ int create_t(PlaneMft* p, const double* x, const double* y, const double* u, con
     auto layout = [&](Carver& c) {
         for (int d = 0; d < (own_adjoint ? 3 : 2); ++d) {
             const Dims q = dims_of(p, d);
-            auto mat = [&](PlaneMat& m, int columns, int K) {
-                m.digits = takes_digits(K, q.longest());
+            auto mat = [&](PlaneMat& m, int columns, int K, bool digits) {
+                m.digits = digits;
                 with_form<T>(m.digits, [&](auto f) { carve_mat<decltype(f)>(c, m, 2 * round_up(columns, 8), columns, K); });
             };
-            mat(p->rgt[d], q.C, q.K2);
-            mat(p->lft[d], q.R, q.K1);
+            mat(p->rgt[d], q.C, q.K2, q.digits(false));
+            mat(p->lft[d], q.R, q.K1, q.digits(true));
         }
         auto weights = [&](const double* w, int n) { return w ? c.take(sizeof(T) * (size_t)n) : nullptr; };
         p->wk2[HX_FORWARD] = weights(wx, p->nx);
