@@ -355,6 +355,7 @@ struct Carver {
 //   512^2                     0.8         2.9           3.0              4.0           3.5
 //   256^2                     0.9         2.8           4.0              5.3           3.5
 //   400^2                     1.1         2.6           3.0              3.5           2.6
+//   700^2                     0.9         2.9                            3.8           3.3
 //   1024^2                    1.2                                        3.7           4.6
 //   (the step, 64 of 512^2)  4.7 ms       4.5           4.2              3.8            13
 // Images of Lyot coronagraphs (511^2 to 700^2 pupils) are off by 1.0-5.9, 5.0-6.8, 5.5-6.6, 7.6-10 and 14-24, and a pass over
